@@ -118,6 +118,8 @@ class KernelPlan:
             kind = "merge_path_seq_gather4"
         d = {"kind": kind, "items_per_unit": self.items_per_unit, "n_tile": self.n_tile,
              "snap": self.snap, "n_units": self.n_units}
+        if self.flags & nat.PLAN_WALK:
+            d["form"] = "walk"
         if self.grid_blocks:
             d["grid_blocks"] = self.grid_blocks
         return d
@@ -306,13 +308,25 @@ def seq_items_per_unit(stats):
     return _pow2_clamp(items / (SM_COUNT * SEQ_WARPS_PER_SM * 2), 128, 1024)
 
 
+WALK_WARPS_PER_SM = 24  # resident warps of the range-walk SpMM kernel (6 CTAs of 4)
+
+
+def walk_items_per_unit(n_rows, nnz):
+    """Merge-path unit size for the range-walk SpMM kernel: one wave of its
+    resident warps, between 128 and 1024 items (power-law matrix, N = 64: 128
+    items 105 us, 256 88, 512 85, 1024 81; 100000 rows of 4, N = 32: 128 and
+    256 items 20 us, 512 24)."""
+    return _pow2_clamp((int(n_rows) + int(nnz)) / (SM_COUNT * WALK_WARPS_PER_SM), 128, 1024)
+
+
 def default_spmm_plan(stats, n_dense, dtype, row_cap=0):
     """Heuristic SpMM plan: the batched merge-path kernel (nonzero-balanced
     units, rows split across units where long); row groups when a per-row
     segment cap is requested."""
     if row_cap > 0 or stats.n_rows == 0:
         return KernelPlan(nat.ALGO_ROWS, lanes=32, row_cap=row_cap)
-    return KernelPlan(nat.ALGO_SEQ, items_per_unit=seq_items_per_unit(stats), snap=SPMM_SNAP_DEFAULT)
+    return KernelPlan(nat.ALGO_SEQ, items_per_unit=seq_items_per_unit(stats), snap=SPMM_SNAP_DEFAULT,
+                      flags=nat.PLAN_WALK)
 
 
 # How the prepared SpMM paths pick their plan: "learned" (the shipped

@@ -21,7 +21,7 @@
 // kernels (:778-919), the alg2 kernels (spmm_csr_opt_alg2.py:338-629) and the
 // COO row-run kernels (spmm_coo.py:135-241).
 #include "fsb_spmm_common.cuh"
-#include "fsb_spmm_seq.cuh"
+#include "fsb_spmm_walk.cuh"
 
 namespace fsb {
 
@@ -505,6 +505,21 @@ extern "C" int fsb_spmm_csr(const fsb_csr* A, const void* B, int64_t ldb, int64_
     if (plan->algo == FSB_ALGO_GATHER)
         return spmm_gather_dispatch(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes,
                                     st);
+    if (plan->algo == FSB_ALGO_SEQ && (plan->flags & FSB_PLAN_WALK) && !(plan->flags & FSB_PLAN_TMA_GATHER) &&
+        walk_takes(A, ldb, ldc, out_dtype, acc_mode)) {
+        switch (A->value_dtype) {
+        case FSB_F16: return walk_dispatch_f16(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
+        case FSB_BF16: return walk_dispatch_bf16(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
+        case FSB_F32: return walk_dispatch_f32(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
+        case FSB_F64: return walk_dispatch_f64(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
+        case FSB_C32: return walk_dispatch_c32(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
+        case FSB_C64: return walk_dispatch_c64(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
+        case FSB_C128: return walk_dispatch_c128(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
+        default:
+            fsb_host::set_error("fsb_spmm_csr: value dtype code %d", A->value_dtype);
+            return FSB_ERR_UNSUPPORTED;
+        }
+    }
     if (plan->algo == FSB_ALGO_SEQ) {
         switch (A->value_dtype) {
         case FSB_F16: return seq_dispatch_f16(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);

@@ -62,7 +62,8 @@ def _merge(items, snap):
 
 
 def _seq(items, n_tile=0):
-    return lambda: _plan.KernelPlan(nat.ALGO_SEQ, items_per_unit=items, n_tile=n_tile, snap=_plan.SPMM_SNAP_DEFAULT)
+    return lambda: _plan.KernelPlan(nat.ALGO_SEQ, items_per_unit=items, n_tile=n_tile, snap=_plan.SPMM_SNAP_DEFAULT,
+                                    flags=nat.PLAN_WALK)
 
 
 # (name, plan factory); the order is the network's output order.
@@ -275,6 +276,32 @@ def targets_from_times(times):
 
 
 # ---------------------------------------------------------------- selector
+# Row-group picks stay below this many path items (rows + nonzeros); above it
+# the range-walk kernel is the faster one.  Measured on 200 held-out (matrix,
+# N) pairs with a row-group pick, walk time over row-group time: 1.2 - 1.3 at
+# 10^4 rows (launch bound), 1.0 at 0.5 - 1.5 M items, 0.87 at 2 - 10 M, 0.63 -
+# 0.8 above.
+ROW_GROUP_MAX_ITEMS = 1 << 20
+
+
+def fit_to_walk(plan, n_rows, nnz, acc_mode):
+    """The selector's CUDA-core pick in the range-walk kernel's terms.  The
+    network's candidates were timed with the earlier merge-path form, whose
+    best units were smaller: a merge-path pick keeps its column tile and takes
+    its unit size from ``walk_items_per_unit`` (held-out power-law matrices:
+    1.12 x the best candidate with the pick's own units, 1.06 x with these),
+    and a large row-group or plain merge pick becomes the range walk.
+    Compensated sums run in the earlier form and keep the pick."""
+    if acc_mode == nat.ACC_COMP or isinstance(plan, _plan.BsrPlan):
+        return plan
+    items = _plan.walk_items_per_unit(n_rows, nnz)
+    if plan.flags & nat.PLAN_WALK:
+        plan.items_per_unit = items
+    elif n_rows + nnz >= ROW_GROUP_MAX_ITEMS:
+        return _seq(items)()
+    return plan
+
+
 class LearnedSelector:
     """Selector network with its feature standardisation; falls back to the
     autotuner outside the training range or on a near tie."""
@@ -332,7 +359,7 @@ class LearnedSelector:
                 return plan
         if confident:
             self.last = ("learned", CANDIDATE_NAMES[k])
-            return SPMM_CANDIDATES[k][1]()
+            return fit_to_walk(SPMM_CANDIDATES[k][1](), int(n_rows), int(data.numel()), acc_mode)
         plan, _ = self.autotuner.tune(data, indices, indptr, n_rows, n_cols, B, C, acc_mode)
         self.last = ("autotune", plan.describe())
         return plan

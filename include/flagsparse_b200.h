@@ -90,6 +90,13 @@ extern "C" {
                                   gap of back-to-back SpMVs (solver loops,
                                   CUDA graphs); results are unchanged       */
 
+#define FSB_PLAN_WALK 4        /* SEQ: each sub-group of a warp walks its own
+                                  contiguous part of the unit's nonzeros (staged
+                                  in shared memory with their rows) and stores
+                                  its rows itself; calls it does not take
+                                  (compensated accumulators, more than 2^32
+                                  columns) run in the plain SEQ form          */
+
 /* A CSR matrix (or a sorted COO matrix seen as row runs).
  * row_ptr has n_rows + 1 entries.  If row_map is non-null, row r of this
  * structure is written to output row row_map[row_ptr[r]] (COO row runs:

@@ -1,0 +1,83 @@
+"""The range-walk form of the batched merge-path SpMM (FSB_PLAN_WALK) against
+the FP64 oracle where it can go wrong: rows at the edges of batches (8), chunks
+(256), units and sub-group ranges, ranges without a nonzero, rows that end
+where a unit begins, runs of empty rows, and every lane layout (whole 16-byte
+lane vectors and strided columns of odd widths).
+
+Bounds (condition-scaled, tests/numerics.py): those of the other SpMM forms;
+n products summed in float32 err by at most about n * 2^-24 of their
+magnitude, 3e-5 for the longest row here (300 in a chain of 8 + 300 / 8)."""
+
+import pytest
+import torch
+
+from flagsparse_public_b200 import _native as nat
+from flagsparse_public_b200 import _plan
+from oracle import oracle as orc
+from tests.gpu_cases import csr_from_lengths, dense
+from tests.numerics import REL_BOUND, scaled_error
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+PATTERNS = {
+    "few": [2, 0, 1],
+    "single": [1],
+    "batch_edges": [7, 8, 9, 1, 16, 15, 17, 0, 8],
+    "chunk_edges": [255, 1, 256, 257, 0, 511, 2, 300],
+    "unit_start_end": [100, 100, 64, 36, 0, 0, 0, 200],
+    "ones": [1] * 300,
+    "empty_runs": [0] * 70 + [5] + [0] * 40 + [3, 0, 290] + [0] * 33,
+}
+MODES = [(torch.float32, nat.ACC_NATIVE, torch.float32, 3e-5),
+         (torch.float32, nat.ACC_WIDE, torch.float32, REL_BOUND[torch.float32]),
+         (torch.float64, nat.ACC_NATIVE, torch.float64, REL_BOUND[torch.float64]),
+         (torch.bfloat16, nat.ACC_NATIVE, torch.float32, 3e-5),
+         (torch.complex128, nat.ACC_NATIVE, torch.complex128, REL_BOUND[torch.complex128])]
+
+
+def _id(m):
+    return f"{str(m[0])[6:]}-{['native', 'wide'][m[1]]}"
+
+
+@pytest.mark.parametrize("pattern", sorted(PATTERNS))
+@pytest.mark.parametrize("mode", MODES, ids=_id)
+def test_walk_matches_oracle(pattern, mode):
+    dtype, acc, out_dtype, bound = mode
+    wide_idx = pattern in ("ones", "chunk_edges")  # 64-bit columns with 32-bit offsets on two patterns
+    data, indices, indptr, (n_rows, n_cols) = csr_from_lengths(
+        PATTERNS[pattern], 600, seed=61, dtype=dtype, index_dtype=torch.int64 if wide_idx else torch.int32,
+        ptr_dtype=torch.int32 if wide_idx else torch.int64)
+    d = (data.to(DEV), indices.to(DEV), indptr.to(DEV))
+    for n_dense in (1, 3, 5, 16, 33, 40, 64, 100, 130):
+        B = dense((n_cols, n_dense), 62, dtype)
+        exact, mag = orc.spmm_csr_exact(data, indices, indptr, B)
+        Bd = B.to(DEV)
+        for items, snap, n_tile, grid in ((16, 0, 0, 0), (100, 0, 0, 0), (256, 64, 0, 0), (2048, 64, 0, 1), (77, 0, 8, 2)):
+            plan = _plan.KernelPlan(nat.ALGO_SEQ, items_per_unit=items, snap=snap, n_tile=n_tile, grid_blocks=grid,
+                                    flags=nat.PLAN_WALK)
+            out = []
+            for finish_in_kernel in (True, False):
+                C = torch.full((n_rows, n_dense), float("nan"), dtype=out_dtype, device=DEV)
+                if not finish_in_kernel:
+                    plan.runs = False  # split rows finished by the fix-up kernel: the same sums
+                _plan.run_spmm(*d, n_rows, n_cols, Bd, C, acc, plan)
+                out.append(C)
+            assert torch.equal(out[0], out[1]), (n_dense, items)
+            assert scaled_error(out[0], exact, mag) <= bound, (n_dense, items, n_tile)
+
+
+def test_walk_leaves_non_finite_b_rows_alone():
+    """Lanes without a nonzero in a ragged batch touch no B row: infinities
+    and NaN in rows that no nonzero names stay out of the result."""
+    data, indices, indptr, (n_rows, n_cols) = csr_from_lengths([3, 0, 5, 1], 64, seed=63)
+    B = dense((n_cols, 64), 64, torch.float32)
+    used = torch.zeros(n_cols, dtype=torch.bool)
+    used[indices.long()] = True
+    B[~used] = float("nan")
+    B[0 if not used[0] else int((~used).nonzero()[0])] = float("inf")
+    exact, mag = orc.spmm_csr_exact(data, indices, indptr, torch.where(used[:, None], B, torch.zeros_like(B)))
+    C = torch.empty((n_rows, 64), device=DEV)
+    _plan.run_spmm(data.to(DEV), indices.to(DEV), indptr.to(DEV), n_rows, n_cols, B.to(DEV), C, nat.ACC_NATIVE,
+                   _plan.KernelPlan(nat.ALGO_SEQ, items_per_unit=128, flags=nat.PLAN_WALK))
+    assert scaled_error(C, exact, mag) <= 3e-5
