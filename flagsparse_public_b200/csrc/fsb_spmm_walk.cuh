@@ -117,6 +117,7 @@ k_spmm_walk(const V* __restrict__ val, const I* __restrict__ col, const void* __
     __shared__ __align__(16) V sm_val[kWarps][CH];
     __shared__ __align__(16) uint32_t sm_brk[kWarps][WORDS];  // bit per nonzero: a row starts here
     __shared__ __align__(16) A sm_head[kSpmmThreads][VW];  // a range's first row, finished before its part from earlier
+    __shared__ __align__(16) A sm_open[kSpmmThreads][VW];  // the open row's sum before the chunk (first sub-group's lanes)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t* s_col = sm_col[warp];
     int* s_row = sm_row[warp];
@@ -198,6 +199,10 @@ k_spmm_walk(const V* __restrict__ val, const I* __restrict__ col, const void* __
         // a continued row that ends where the unit begins: nothing left to add
         if (continued && n_ends > 0 && start_of(1) == 0 && sub == 0 && col_ok) put_partial(head_val, unit, acc);
 
+        if (sub == 0) {
+#pragma unroll
+            for (int w = 0; w < VW; ++w) sm_open[threadIdx.x][w] = acc[w];
+        }
         int rb = 0;        // rows whose start has been passed
         int open_row = 1;  // row open at the chunk's start
         for (int kc = 0;; kc += CH) {
@@ -265,20 +270,18 @@ k_spmm_walk(const V* __restrict__ val, const I* __restrict__ col, const void* __
                     else return (uint32_t)(s_brk[e >> 3] >> (e & 4)) & 15u;
                 };
                 // the range's first row began before it (cont: and is not finished yet)
-                bool joined, cont;
-                int rcur = kc > 0 || continued ? open_row : 0;  // 0: no row open yet
-                uint32_t first_mask = ~0u;  // the first nonzero of a range ends nothing
-                if (sub > 0 || kc == 0) {
+                const bool has_open = kc > 0 || continued;
+                bool joined = true;
+                int rcur = has_open ? open_row : 0;  // 0: no row open yet
+                uint32_t first_mask = ~0u;
+                if (sub > 0 || !has_open) {
                     const bool starts = some && (brk_bits(e_lo) & 1u);
                     joined = !starts;
                     if (starts) rcur = s_row[e_lo];
-                    first_mask = ~1u;
-                    cont = joined;
-                } else {
-                    joined = true;
-                    cont = continued && open_row == 1;
+                    first_mask = ~1u;  // the first nonzero of a range ends nothing
                 }
-                const bool cont0 = cont;
+                bool cont = joined;
+                zero_acc<A, VW>(acc);
                 auto batch = [&](int e, int cnt, bool whole) {
                     vec_t<V, VW> bv[U];
                     if (whole) {
@@ -345,7 +348,15 @@ k_spmm_walk(const V* __restrict__ val, const I* __restrict__ col, const void* __
 
                 // ---- the sub-groups' open partials, in order: f = the tail
                 // holds no part of the previous sub-group's row
-                const bool broke = cont0 && !cont;
+                const bool broke = joined && !cont;
+                if (sub == 0 && has_open) {  // the chunk's sum joins the open row's once
+#pragma unroll
+                    for (int w = 0; w < VW; ++w) {
+                        const A o = sm_open[threadIdx.x][w];
+                        if (broke) sm_head[threadIdx.x][w] = acc_add(o, sm_head[threadIdx.x][w]);
+                        else acc[w] = acc_add(o, acc[w]);
+                    }
+                }
                 int f = (sub > 0 && joined && !broke) ? 0 : 1;
                 int row_t = rcur;
 #pragma unroll
@@ -374,21 +385,22 @@ k_spmm_walk(const V* __restrict__ val, const I* __restrict__ col, const void* __
                             h[w] = sm_head[threadIdx.x][w];
                             if (sub > 0) h[w] = acc_add(in[w], h[w]);
                         }
-                        finish(sub > 0 ? in_row : 1, h);
+                        finish(sub > 0 ? in_row : open_row, h);
                     }
                     const int next_joined = __shfl_down_sync(full, (int)joined, LPN);
                     if (sub < NPAR - 1 && !next_joined && row_t > 0) finish(row_t, acc);
                     // the open row's partial moves to the first sub-group
 #pragma unroll
-                    for (int w = 0; w < VW; ++w) {
-                        const A t = shfl_idx(full, acc[w], (32 - LPN) + lig, 32);
-                        acc[w] = sub == 0 ? t : A{};
-                    }
+                    for (int w = 0; w < VW; ++w) acc[w] = shfl_idx(full, acc[w], (32 - LPN) + lig, 32);
                 } else if (broke) {
                     A h[VW];
 #pragma unroll
                     for (int w = 0; w < VW; ++w) h[w] = sm_head[threadIdx.x][w];
-                    finish(1, h);
+                    finish(open_row, h);
+                }
+                if (sub == 0) {
+#pragma unroll
+                    for (int w = 0; w < VW; ++w) sm_open[threadIdx.x][w] = acc[w];
                 }
                 open_row = __shfl_sync(full, row_t, 31);
                 __syncwarp();  // the next chunk overwrites the staged one
