@@ -280,24 +280,41 @@ def _vec_elems(dtype):
     return max(1, 16 // dtype.itemsize)
 
 
+SM_COUNT = 148  # B200
+
+
+def spmv_row_lanes(n_rows, mean, vec, skewed):
+    """Lanes per row of the row-group SpMV (the rule and its measurements:
+    spmv_row_lanes in csrc/fsb_spmv.cu, which one-shot calls use)."""
+    if skewed:
+        return _pow2_clamp(2 * mean / vec, 2, 32)
+    lanes = 2 if mean < 12.0 else 4
+    while lanes < 32 and n_rows * lanes * 2 <= SM_COUNT * 1024 and 2.0 * lanes * vec <= 2.0 * mean:
+        lanes *= 2
+    return lanes
+
+
+def spmv_merge_items(n_rows, nnz):
+    """Merge-path SpMV unit: (rows + nonzeros) over 16 warps per SM, 128 to
+    1024 items (spmv_merge_items in csrc/fsb_spmv.cu)."""
+    return _pow2_clamp((n_rows + nnz) / (SM_COUNT * 16), SPMV_MERGE_THREADS, 1024)
+
+
 def default_spmv_plan(stats, dtype, row_cap=0):
-    """Heuristic SpMV plan: merge path for skewed rows that are short on
-    average, else row groups sized so a row's nonzeros take about half a
-    16-byte vector per lane (more lanes shorten each row's dependent load
-    chain; long average rows keep 16-32 lanes busy even when a few rows are
-    much longer: measured faster than merge path there)."""
+    """Heuristic SpMV plan: merge path for skewed rows of less than 128
+    nonzeros on average (longer average rows keep 16-32 lanes busy even when a
+    few rows are much longer), else row groups of few lanes.  The same choice
+    as checked_plan in csrc/fsb_spmv.cu."""
     if row_cap > 0 or stats.n_rows == 0:
         lanes = _pow2_clamp(stats.mean_row / _vec_elems(dtype), 2, 32) if stats.n_rows else 32
         return KernelPlan(nat.ALGO_ROWS, lanes=lanes, row_cap=row_cap)
     skewed = stats.max_row > 8 * max(stats.mean_row, 1.0) + 256
-    if skewed and stats.mean_row < 32:
-        ipt = 8 if dtype.itemsize <= 4 else 4
-        return KernelPlan(nat.ALGO_MERGE, items_per_unit=SPMV_MERGE_THREADS * ipt)
-    lanes = _pow2_clamp(2 * stats.mean_row / _vec_elems(dtype), 2, 32)
+    if skewed and stats.mean_row < 128.0:
+        return KernelPlan(nat.ALGO_MERGE, items_per_unit=spmv_merge_items(stats.n_rows, stats.nnz))
+    lanes = spmv_row_lanes(stats.n_rows, stats.mean_row, _vec_elems(dtype), skewed)
     return KernelPlan(nat.ALGO_ROWS, lanes=lanes, flags=nat.PLAN_OVERLAP_LAUNCH)
 
 
-SM_COUNT = 148  # B200
 SEQ_WARPS_PER_SM = 32
 
 

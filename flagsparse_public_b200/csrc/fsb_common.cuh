@@ -261,6 +261,11 @@ __device__ __forceinline__ c128_t shfl_idx(unsigned m, c128_t v, int src, int w)
     return c128_t{__shfl_sync(m, v.re, src, w), __shfl_sync(m, v.im, src, w)};
 }
 
+template <>
+__device__ __forceinline__ comp_t shfl_idx(unsigned m, comp_t v, int src, int w) {
+    return comp_t{__shfl_sync(m, v.s, src, w), __shfl_sync(m, v.c, src, w)};
+}
+
 // Reduce across a power-of-two segment of `width` lanes (xor butterfly over
 // offsets first..width/2).  All lanes of the segment end with the total.
 template <class A>

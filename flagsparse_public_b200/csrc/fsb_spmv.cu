@@ -5,13 +5,12 @@
 //                    warp-per-row), 128-bit streaming loads of values and column
 //                    indices on the aligned body of each row, read-only cached
 //                    gathers of x, xor-butterfly reduction inside the group.
-//   * k_spmv_merge : merge-path tiles over the (row ends + nonzeros) path
-//                    (Merrill & Garland, SC'16): every CTA gets the same number
-//                    of path items whatever the row-length skew.  Products are
-//                    staged in shared memory, each thread walks its stretch of
-//                    the path, a warp-shuffle segmented scan carries partial
-//                    rows across threads, and rows that cross tile boundaries
-//                    are finished by k_spmv_merge_fixup from per-tile carries.
+//   * k_spmv_merge : merge-path units of equal (row ends + nonzeros) whatever
+//                    the row-length skew (Merrill & Garland, SC'16), a warp per
+//                    unit.  Each lane sums 8 consecutive nonzeros in order and
+//                    stores the rows that lie inside them; one segmented warp
+//                    scan per 256 nonzeros joins the lanes' open sums.  Rows
+//                    that cross units are finished by k_spmv_merge_fixup.
 //
 // FlagSparse computes the same products in _spmv_csr_real_kernel
 // (spmv_csr.py:158-184), _spmv_csr_complex_kernel (:187-219), the CSR-vector
@@ -33,35 +32,75 @@ constexpr int kMergeMaxTile = kMergeThreads * kMergeMaxItemsPerThread;
 // of this kernel would need)
 constexpr int64_t kOverlapMaxBlocks = 148 * 4;
 
-// Partial sum of row nonzeros [s, e) handled by `lane` of a T-lane group.
-// VEC-wide aligned body, scalar head and tail.
+// The nonzeros [kb, kb + VEC) of the streams, kb a multiple of VEC: 16-byte
+// loads where the whole vector lies inside the arrays (the last one of the
+// matrix may not), single elements otherwise.
+template <class V, class I, int VEC>
+__device__ __forceinline__ void load_chunk(const V* __restrict__ val, const I* __restrict__ col, int64_t kb,
+                                           int64_t nnz, vec_t<V, VEC>& vv, vec_t<I, VEC>& cc) {
+    if (kb + VEC <= nnz) {
+        vv = ld_stream<V, VEC>(val + kb);
+        cc = ld_stream<I, VEC>(col + kb);
+    } else {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            vv.v[j] = vzero<V>();
+            cc.v[j] = 0;
+            if (kb + j < nnz) {
+                vv.v[j] = ld_stream1(val + kb + j);
+                cc.v[j] = ld_stream1(col + kb + j);
+            }
+        }
+    }
+}
+
+// Partial sum of row nonzeros [s, e) handled by `lane` of a T-lane group: the
+// aligned VEC-wide chunks covering the row, the elements outside it skipped.
+// One loop and one chain of loads per row (chunk, x) where a scalar head, an
+// aligned body and a scalar tail made three; two chunks per lane in flight.
+// What bounds it is the loads of x (about one line per cycle and SM) and, for
+// short rows, the chain of loads per row: few lanes per row with a whole
+// chunk each beat many (see spmv_row_lanes).
 template <class V, class A, class I>
 __device__ __forceinline__ A row_partial(const V* __restrict__ val, const I* __restrict__ col,
-                                         const V* __restrict__ x, int64_t s, int64_t e,
+                                         const V* __restrict__ x, int64_t s, int64_t e, int64_t nnz,
                                          int lane, int T, bool vec_ok) {
     constexpr int VV = VecWidth<V>::value;
     constexpr int VI = VecWidth<I>::value;
     constexpr int VEC = VV < VI ? VV : VI;
     A acc = Acc<V, A>::zero();
     if (VEC > 1 && vec_ok) {
-        int64_t a0 = (s + VEC - 1) & ~(int64_t)(VEC - 1);
-        if (a0 > e) a0 = e;
-        int64_t a1 = e & ~(int64_t)(VEC - 1);
-        if (a1 < a0) a1 = a0;
-        for (int64_t k = s + lane; k < a0; k += T)
-            acc = Acc<V, A>::fma(ld_stream1(val + k), ld_ro1(x + idx(ld_stream1(col + k))), acc);
-#pragma unroll 2
-        for (int64_t kb = a0 + (int64_t)lane * VEC; kb < a1; kb += (int64_t)T * VEC) {
-            vec_t<V, VEC> vv = ld_stream<V, VEC>(val + kb);
-            vec_t<I, VEC> cc = ld_stream<I, VEC>(col + kb);
-            V xv[VEC];
+        for (int64_t kb = (s & ~(int64_t)(VEC - 1)) + (int64_t)lane * VEC; kb < e; kb += 2 * (int64_t)T * VEC) {
+            const int64_t k2 = kb + (int64_t)T * VEC;
+            const bool two = k2 < e;
+            vec_t<V, VEC> v0, v1;
+            vec_t<I, VEC> c0, c1;
+            V x0[VEC], x1[VEC];
+            load_chunk<V, I, VEC>(val, col, kb, nnz, v0, c0);
+            if (two) load_chunk<V, I, VEC>(val, col, k2, nnz, v1, c1);
 #pragma unroll
-            for (int j = 0; j < VEC; ++j) xv[j] = ld_ro1(x + idx(cc.v[j]));
+            for (int j = 0; j < VEC; ++j)
+                if (kb + j >= s && kb + j < e) x0[j] = ld_ro1(x + idx(c0.v[j]));
+            if (two) {
 #pragma unroll
-            for (int j = 0; j < VEC; ++j) acc = Acc<V, A>::fma(vv.v[j], xv[j], acc);
+                for (int j = 0; j < VEC; ++j)
+                    if (k2 + j < e) x1[j] = ld_ro1(x + idx(c1.v[j]));
+            }
+            // four short chains, then their sum: a lane with several chunks
+            // rounds no more often than many lanes with one each
+            A t[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) t[q] = Acc<V, A>::zero();
+#pragma unroll
+            for (int j = 0; j < VEC; ++j)
+                if (kb + j >= s && kb + j < e) t[j & 1] = Acc<V, A>::fma(v0.v[j], x0[j], t[j & 1]);
+            if (two) {
+#pragma unroll
+                for (int j = 0; j < VEC; ++j)
+                    if (k2 + j < e) t[2 + (j & 1)] = Acc<V, A>::fma(v1.v[j], x1[j], t[2 + (j & 1)]);
+            }
+            acc = acc_add(acc, acc_add(acc_add(t[0], t[1]), acc_add(t[2], t[3])));
         }
-        for (int64_t k = a1 + lane; k < e; k += T)
-            acc = Acc<V, A>::fma(ld_stream1(val + k), ld_ro1(x + idx(ld_stream1(col + k))), acc);
     } else {
 #pragma unroll 4
         for (int64_t k = s + lane; k < e; k += T)
@@ -77,7 +116,8 @@ template <class V, class A, class O, class I, class P>
 __global__ void __launch_bounds__(kRowsThreads)
 k_spmv_rows(const V* __restrict__ val, const I* __restrict__ col, const P* __restrict__ ptr,
             const I* __restrict__ row_map, const V* __restrict__ x, O* __restrict__ y,
-            int64_t n_rows, int64_t row_cap, int64_t comp_threshold, int lanes_log2, int vec_ok, int overlap) {
+            int64_t n_rows, int64_t nnz, int64_t row_cap, int64_t comp_threshold, int lanes_log2, int vec_ok,
+            int overlap) {
     // programmatic dependent launch: wait until the previous kernel on the
     // stream has completed and its writes are visible -- nothing is read
     // before -- and let the next launch start once this CTA's rows are done
@@ -95,12 +135,12 @@ k_spmv_rows(const V* __restrict__ val, const I* __restrict__ col, const P* __res
         A acc;
         if constexpr (is_comp<A>::value) {
             if (e - s > comp_threshold) {
-                acc = row_partial<V, comp_t, I>(val, col, x, s, e, lane, T, vec_ok);
+                acc = row_partial<V, comp_t, I>(val, col, x, s, e, nnz, lane, T, vec_ok);
             } else {
-                acc = comp_t{row_partial<V, float, I>(val, col, x, s, e, lane, T, vec_ok), 0.f};
+                acc = comp_t{row_partial<V, float, I>(val, col, x, s, e, nnz, lane, T, vec_ok), 0.f};
             }
         } else {
-            acc = row_partial<V, A, I>(val, col, x, s, e, lane, T, vec_ok);
+            acc = row_partial<V, A, I>(val, col, x, s, e, nnz, lane, T, vec_ok);
         }
         acc = segment_reduce(mask, acc, 1, T);
         if (lane == 0) {
@@ -112,112 +152,182 @@ k_spmv_rows(const V* __restrict__ val, const I* __restrict__ col, const P* __res
 }
 
 // ---------------------------------------------------------- merge path ----
-// unit_coords[2u], [2u+1] = (rows ended, nonzeros consumed) at the start of tile u.
-// Scratch per tile: carry_row (row still open at the tile end, -1 if none),
-// carry_val (its partial), head_val (partial of the tile's first finished row
-// when that row began in an earlier tile).
+// unit_coords[2u], [2u+1] = (rows ended, nonzeros consumed) at the start of unit u.
+// Scratch per unit: carry_row (row still open at the unit end, -1 if none),
+// carry_val (its partial), head_val (partial of the unit's first finished row
+// when that row began in an earlier unit).
+//
+// What bounds it: the random loads of x.  Each lane's load of x is its own
+// line, and an SM takes about one line per cycle: 24 M nonzeros cost 84 us on
+// 148 SMs.  A CTA per 512- or 1024-item tile (products in shared memory, a
+// binary search and a serial walk per thread, two barriers) kept loads in
+// flight a third of the time; with a warp per unit nothing waits for other
+// warps.  Zipf rows, 24 M nonzeros over 1.5 M rows: float64 354 -> 146 us,
+// float32 137 -> 122, float32 with float64 sums 268 -> 125; 0.8 M rows of
+// 40 (12 M nonzeros, skewed): warp-per-row groups 230, this form 62.  Loading
+// the next chunk's columns and row offsets a chunk ahead: 150 us (float64).
+// 8 resident CTAs (64 registers) for values below 8 bytes, 6 (80) else: 173 us
+// with 8 for float64.
+// N consecutive elements from an address that is a multiple of 16 bytes (or of
+// the N elements where those are fewer bytes), in streaming vector loads.
+template <class T, int N>
+__device__ __forceinline__ void load_group(const T* p, T (&out)[N]) {
+    constexpr int M = (int)sizeof(T) * N <= 16 ? N : 16 / (int)sizeof(T);
+#pragma unroll
+    for (int i = 0; i < N; i += M) {
+        const vec_t<T, M> t = ld_stream<T, M>(p + i);
+#pragma unroll
+        for (int j = 0; j < M; ++j) out[i + j] = t.v[j];
+    }
+}
+
 template <class V, class A, class O, class I, class P>
-__global__ void __launch_bounds__(kMergeThreads)
+__global__ void __launch_bounds__(kMergeThreads, sizeof(V) >= 8 ? 6 : 8)
 k_spmv_merge(const V* __restrict__ val, const I* __restrict__ col, const P* __restrict__ ptr,
              const I* __restrict__ row_map, const V* __restrict__ x, O* __restrict__ y,
-             int64_t n_rows, const int64_t* __restrict__ coords, int items_per_thread,
+             int64_t n_rows, int64_t nnz, int vec_ok, const int64_t* __restrict__ coords, int64_t n_units,
              int64_t* __restrict__ carry_row, A* __restrict__ carry_val, A* __restrict__ head_val) {
-    __shared__ A s_prod[kMergeMaxTile];
-    __shared__ int s_end[kMergeMaxTile];
-    __shared__ A s_wv[kMergeThreads / 32];
-    __shared__ int s_wf[kMergeThreads / 32];
-
-    const int64_t tile = blockIdx.x;
-    const int64_t r0 = coords[2 * tile], k0 = coords[2 * tile + 1];
-    const int64_t r1 = coords[2 * tile + 2], k1 = coords[2 * tile + 3];
-    const int rows_tile = (int)(r1 - r0);  // row ends inside the tile
-    const int nnz_tile = (int)(k1 - k0);
-    const int items = rows_tile + nnz_tile;
-    const int tid = threadIdx.x;
-    // Coordinates that do not come from an unsnapped partition with this tile
-    // size would overrun the shared-memory staging: leave such a tile alone
-    // (uniform across the block, before any barrier).
-    if (r1 < r0 || k1 < k0 || (r1 - r0) + (k1 - k0) > (int64_t)kMergeThreads * items_per_thread) return;
-
-    for (int j = tid; j < nnz_tile; j += kMergeThreads) {
-        const int64_t k = k0 + j;
-        s_prod[j] = Acc<V, A>::fma(ld_stream1(val + k), ld_ro1(x + idx(ld_stream1(col + k))), Acc<V, A>::zero());
-    }
-    for (int i = tid; i < rows_tile; i += kMergeThreads) s_end[i] = (int)(idx(ptr[r0 + i + 1]) - k0);
-    __syncthreads();
-
-    // This thread's stretch of the tile-local path: [d0, d1).
-    const int d0 = min(tid * items_per_thread, items);
-    const int d1 = min(d0 + items_per_thread, items);
-    int lo = max(0, d0 - nnz_tile), hi = min(d0, rows_tile);
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (s_end[mid] <= d0 - mid - 1) lo = mid + 1; else hi = mid;
-    }
-    int i = lo, j = d0 - lo;
-
-    const bool continued = (r0 < n_rows) && (k0 > idx(ptr[r0]));
-    A run = Acc<V, A>::zero(), first = Acc<V, A>::zero();
-    int first_i = -1;
-    bool head = false;
-    for (int d = d0; d < d1; ++d) {
-        if (i < rows_tile && s_end[i] <= j) {
-            if (!head) {
-                head = true;
-                first = run;
-                first_i = i;
-            } else {
-                const int64_t r = r0 + i;
-                const int64_t out_row = row_map ? idx(row_map[idx(ptr[r])]) : r;
-                y[out_row] = Out<O, A>::cvt(run);
-            }
-            run = Acc<V, A>::zero();
-            ++i;
+    constexpr int E = sizeof(V) <= 8 ? 8 : 4;  // nonzeros per lane and chunk
+    constexpr int CH = 32 * E;
+    constexpr int kWarps = kMergeThreads / 32;
+    constexpr unsigned full = 0xffffffffu;
+    constexpr unsigned kAll = (1u << E) - 1u;
+    __shared__ int sm_row[kWarps][CH];  // number of the row that starts at a nonzero (where the flag is set)
+    __shared__ __align__(8) unsigned char sm_flag[kWarps][CH];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t unit = (int64_t)blockIdx.x * kWarps + warp;
+    if (unit >= n_units) return;
+    int* s_row = sm_row[warp];
+    unsigned char* s_flag = sm_flag[warp];
+    // rows are numbered from 1 at the unit's first row, nonzeros from 0 at k0
+    const int64_t r0 = coords[2 * unit], k0 = coords[2 * unit + 1];
+    const int n_ends = (int)(coords[2 * unit + 2] - r0);  // rows ending in the unit
+    const int nk = (int)(coords[2 * unit + 3] - k0);
+    const int n_rel = n_ends + (r0 + n_ends < n_rows ? 1 : 0);
+    // start of row i + 1, clamped to [-1, nk + 1]
+    auto start_of = [&](int i) -> int {
+        const int64_t s = idx(ptr[r0 + i]) - k0;
+        return s < 0 ? -1 : (s > nk ? nk + 1 : (int)s);
+    };
+    const bool continued = n_rel > 0 && start_of(0) < 0;
+    auto put = [&](int rel, A v) {
+        if (rel == 1 && continued) {
+            head_val[unit] = v;
         } else {
-            run = acc_add(run, s_prod[j]);
-            ++j;
+            const int64_t r = r0 + (rel - 1);
+            y[row_map ? idx(row_map[idx(ptr[r])]) : r] = Out<O, A>::cvt(v);
         }
-    }
-
-    // Segmented inclusive scan of (head, run) across the block:
-    // (f1, v1) . (f2, v2) = (f1 | f2, f2 ? v2 : v1 + v2).
-    const int wl = tid & 31, warp = tid >> 5;
-    bool f = head;
-    A v = run;
+    };
+    // Chunks start at multiples of E in the arrays (aligned vector loads); the
+    // first one reaches `lead` nonzeros before the unit.
+    const int lead = (int)(k0 & (E - 1));
+    int rb = 0;                            // rows whose start has been passed
+    int open_row = continued ? 1 : 0;      // row open before the chunk, 0: none
+    A open_acc = Acc<V, A>::zero();        // its sum so far
+    auto valid_of = [&](int g) -> unsigned {  // the lane's nonzeros g .. g + E - 1 that are the unit's
+        const int lo = g < 0 ? -g : 0, hi = nk - g < E ? nk - g : E;
+        return hi > lo ? (kAll >> (E - hi)) & (kAll << lo) : 0u;
+    };
+    auto load = [&](auto* base, int g, unsigned valid, auto& out) {
+        if (vec_ok && valid && k0 + g + E <= nnz) {
+            load_group(base + k0 + g, out);
+        } else {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const A vu = shfl_up(0xffffffffu, v, o);
-        const int fu = __shfl_up_sync(0xffffffffu, (int)f, o);
-        if (wl >= o) {
-            if (!f) v = acc_add(vu, v);
-            f = f || fu;
+            for (int u = 0; u < E; ++u)
+                if ((valid >> u) & 1u) out[u] = ld_stream1(base + k0 + g + u);
         }
-    }
-    if (wl == 31) {
-        s_wv[warp] = v;
-        s_wf[warp] = (int)f;
-    }
-    __syncthreads();
-    A pv = Acc<V, A>::zero();
-    for (int w = 0; w < warp; ++w) pv = s_wf[w] ? s_wv[w] : acc_add(pv, s_wv[w]);
-    const A incl = f ? v : acc_add(pv, v);
-    A excl = shfl_up(0xffffffffu, incl, 1);
-    if (wl == 0) excl = pv;
-
-    if (head) {
-        const A total = acc_add(excl, first);
-        if (first_i == 0 && continued) {
-            head_val[tile] = total;
-        } else {
-            const int64_t r = r0 + first_i;
-            const int64_t out_row = row_map ? idx(row_map[idx(ptr[r])]) : r;
-            y[out_row] = Out<O, A>::cvt(total);
+    };
+    for (int kc = -lead;; kc += CH) {
+        const bool last = kc + CH >= nk;
+        const int g = kc + lane * E;  // the lane's first nonzero
+        const unsigned valid = valid_of(g);
+        V v[E];
+        I c[E];
+        load(val, g, valid, v);
+        load(col, g, valid, c);
+        if constexpr (E == 8) *reinterpret_cast<uint2*>(s_flag + lane * E) = make_uint2(0u, 0u);
+        else *reinterpret_cast<uint32_t*>(s_flag + lane * E) = 0u;
+        __syncwarp();
+        const int end = last ? nk : kc + CH;
+        for (;;) {
+            const int row = rb + lane;
+            const bool in = row < n_rel;
+            const int s = in ? start_of(row) : 0, e = in ? start_of(row + 1) : 0;
+            const bool take = in && (s < end || (last && row < n_ends));
+            if (take && e > s && s >= 0 && s < end) {
+                s_row[s - kc] = row + 1;
+                s_flag[s - kc] = 1;
+            }
+            if (take && e == s && row < n_ends) {  // an empty row
+                const int64_t r = r0 + row;
+                y[row_map ? idx(row_map[idx(ptr[r])]) : r] = Out<O, A>::cvt(Acc<V, A>::zero());
+            }
+            const int cnt = __popc(__ballot_sync(full, take));
+            rb += cnt;
+            if (cnt < 32) break;
         }
+        V xv[E];
+        const bool whole = __all_sync(full, valid == kAll);
+#pragma unroll
+        for (int u = 0; u < E; ++u)
+            if (whole || ((valid >> u) & 1u)) xv[u] = ld_ro1(x + idx(c[u]));
+        __syncwarp();
+        // the lane's nonzeros in order; a flag ends the row before it
+        uint32_t fl[E / 4];
+#pragma unroll
+        for (int i = 0; i < E / 4; ++i) fl[i] = reinterpret_cast<const uint32_t*>(s_flag + lane * E)[i];
+        A acc = Acc<V, A>::zero(), head = Acc<V, A>::zero();
+        int rcur = 0;
+        bool broke = false;
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            if (fl[u / 4] & (1u << (8 * (u % 4)))) {
+                if (broke) put(rcur, acc);
+                else head = acc;
+                broke = true;
+                rcur = s_row[lane * E + u];
+                acc = Acc<V, A>::zero();
+            }
+            if (whole || ((valid >> u) & 1u)) acc = Acc<V, A>::fma(v[u], xv[u], acc);
+        }
+        // lanes in order: the open row's sum enters at lane 0, each lane's tail
+        // passes on to the lanes up to (and into) the next one holding a break
+        if (lane == 0) {
+            if (broke) head = acc_add(open_acc, head);
+            else acc = acc_add(open_acc, acc);
+        }
+        const unsigned breaks = __ballot_sync(full, broke);
+        const unsigned upto = breaks & (0xffffffffu >> (31 - lane));
+        const int seg = upto ? 31 - __clz(upto) : 0;  // the lane whose tail the row began in (lane 0: open_row)
+        const int from = __shfl_sync(full, rcur, seg);
+        const int row_t = upto ? from : open_row;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const A up = shfl_up(full, acc, o);
+            if (lane - o >= seg) acc = acc_add(up, acc);
+        }
+        const A in = shfl_up(full, acc, 1);
+        const int in_row = __shfl_up_sync(full, row_t, 1);
+        if (broke) {
+            const A total = lane > 0 ? acc_add(in, head) : head;
+            const int rel = lane > 0 ? in_row : open_row;
+            if (rel > 0) put(rel, total);
+        }
+        open_acc = shfl_idx(full, acc, 31, 32);
+        open_row = __shfl_sync(full, row_t, 31);
+        __syncwarp();  // flags and rows are overwritten by the next chunk
+        if (last) break;
     }
-    if (tid == kMergeThreads - 1) {
-        const bool open = (r1 < n_rows) && (k1 > idx(ptr[r1]));
-        carry_row[tile] = open ? r1 : -1;
-        if (open) carry_val[tile] = incl;
+    if (lane == 0) {
+        bool open = false;
+        if (nk > 0 && n_rel > n_ends) {
+            const int s1 = start_of(n_ends);
+            open = nk > (s1 > 0 ? s1 : 0);
+        }
+        // (a continued row without a nonzero here ends with an empty head partial)
+        if (open) carry_val[unit] = open_acc;
+        else if (open_row > 0) put(open_row, open_acc);
+        carry_row[unit] = open ? r0 + n_ends : -1;
     }
 }
 
@@ -300,7 +410,7 @@ extern "C" int fsb_spmv_csr(const fsb_csr* A, const void* x, void* y, int out_dt
                     const int overlap = (plan->flags & FSB_PLAN_OVERLAP_LAUNCH) && grid <= kOverlapMaxBlocks;
                     if (!overlap) {
                         k_spmv_rows<V, Ac, O, I, P><<<(unsigned)grid, kRowsThreads, 0, st>>>(
-                            val, col, ptr, rmap, xv, yv, A->n_rows, plan->row_cap, thr, lg, vec_ok, 0);
+                            val, col, ptr, rmap, xv, yv, A->n_rows, A->nnz, plan->row_cap, thr, lg, vec_ok, 0);
                         return fsb_host::check_launch("k_spmv_rows");
                     }
                     cudaLaunchConfig_t cfg = {};
@@ -312,9 +422,9 @@ extern "C" int fsb_spmv_csr(const fsb_csr* A, const void* x, void* y, int out_dt
                     attr[0].val.programmaticStreamSerializationAllowed = 1;
                     cfg.attrs = attr;
                     cfg.numAttrs = 1;
-                    const int64_t nr = A->n_rows, rc_cap = plan->row_cap;
+                    const int64_t nr = A->n_rows, nz = A->nnz, rc_cap = plan->row_cap;
                     const cudaError_t e = cudaLaunchKernelEx(&cfg, k_spmv_rows<V, Ac, O, I, P>, val, col, ptr, rmap,
-                                                             xv, yv, nr, rc_cap, thr, lg, vec_ok, 1);
+                                                             xv, yv, nr, nz, rc_cap, thr, lg, vec_ok, 1);
                     if (e != cudaSuccess) {
                         fsb_host::set_error("k_spmv_rows (overlapped launch): %s", cudaGetErrorString(e));
                         return FSB_ERR_LAUNCH;
@@ -351,8 +461,9 @@ extern "C" int fsb_spmv_csr(const fsb_csr* A, const void* x, void* y, int out_dt
                     fsb_host::set_error("fsb_spmv_csr: too many merge tiles");
                     return FSB_ERR_LIMIT;
                 }
-                k_spmv_merge<V, Ac, O, I, P><<<(unsigned)n_units, kMergeThreads, 0, st>>>(
-                    val, col, ptr, rmap, xv, yv, A->n_rows, plan->unit_coords, ipt, ms.carry_row,
+                k_spmv_merge<V, Ac, O, I, P><<<(unsigned)ceil_div(n_units, kMergeThreads / 32), kMergeThreads, 0, st>>>(
+                    val, col, ptr, rmap, xv, yv, A->n_rows, A->nnz, aligned16(val) && aligned16(col),
+                    plan->unit_coords, n_units, ms.carry_row,
                     static_cast<Ac*>(ms.carry_val), static_cast<Ac*>(ms.head_val));
                 int rc = fsb_host::check_launch("k_spmv_merge");
                 if (rc) return rc;
@@ -372,26 +483,54 @@ extern "C" int fsb_spmv_csr(const fsb_csr* A, const void* x, void* y, int out_dt
 namespace {
 int64_t check_bytes(const fsb_csr* A) { return align_up(fsb_csr_check_workspace_bytes(A->n_rows, A->nnz), 256); }
 
-// Row-group width / merge-path choice from the check's figures: merge path
-// for skewed rows that are short on average, else 2 * mean / (16-byte vector
-// elements) lanes rounded to a power of two in [2, 32] (ties to even).
+// Lanes of a row group: 2 for rows of less than 12 nonzeros on average, else
+// 4; wider while the whole grid would hold at most 1024 threads per SM and the
+// lanes' chunks stay below twice the row.  Rows that a few long ones dominate
+// (skewed, 128 nonzeros or more on average) take 2 * mean / (16-byte vector
+// elements) lanes.  Measured (us, lanes 2 / 4 / 8 / 16 / 32, float32):
+// 10^6 rows of 4 31 / 45 / 88 / 176 / 359, 10^6 of 8 44 / 58 / 97 / 190 / 390,
+// 10^5 of 23 15 / 13 / 14 / 20 / 38, 5 * 10^5 of 48 113 / 106 / 112 / 142 /
+// 226, 10^5 of 128 48 / 38 / 47 / 54 / 65, 16384 of 16 4.2 / 3.6 / 3.4 / 4.8 /
+// 7.9 (default_spmv_plan in _plan.py follows the same rule).
+int spmv_row_lanes(int64_t n_rows, double mean, int vec, bool skewed) {
+    if (skewed) {
+        double v = 2.0 * mean / vec;
+        if (v < 1.0) v = 1.0;
+        const int lanes = 1 << (int)std::nearbyint(std::log2(v));
+        return lanes < 2 ? 2 : (lanes > 32 ? 32 : lanes);
+    }
+    int lanes = mean < 12.0 ? 2 : 4;
+    while (lanes < 32 && n_rows * lanes * 2 <= 148 * 1024 && 2.0 * lanes * vec <= 2.0 * mean) lanes *= 2;
+    return lanes;
+}
+
+// Merge-path unit: (rows + nonzeros) over 16 warps per SM, 128 to 1024 items
+// (Zipf rows, 256 / 512 / 1024 items: 0.18 M items 8.1 / 9.9 / 13.6 us, 1.2 M
+// 15.9 / 13.3 / 15.3, 3.4 M 27 / 25 / 23, 25 M 154 / 131 / 125).
+int32_t spmv_merge_items(const fsb_csr* A) {
+    double v = (double)(A->n_rows + A->nnz) / (148.0 * 16.0);
+    if (v < 1.0) v = 1.0;
+    const int64_t items = (int64_t)1 << (int)std::nearbyint(std::log2(v));
+    return (int32_t)(items < 128 ? 128 : (items > 1024 ? 1024 : items));
+}
+
+// Row groups or merge path from the check's figures: merge path for skewed
+// rows (the longest above 8 times the mean + 256) of less than 128 nonzeros
+// on average (Zipf rows of 40: row groups 227 us, merge path 61).
 void checked_plan(const fsb_csr* A, const int64_t* fig, fsb_plan* plan) {
     memset(plan, 0, sizeof(*plan));
     const int esz = elem_size(A->value_dtype);
     const int vec = esz >= 16 ? 1 : 16 / esz;
     const double mean = A->n_rows ? (double)A->nnz / (double)A->n_rows : 0.0;
     const bool skewed = (double)fig[5] > 8.0 * (mean > 1.0 ? mean : 1.0) + 256.0;
-    if (A->n_rows > 0 && skewed && mean < 32.0) {
+    if (A->n_rows > 0 && skewed && mean < 128.0) {
         plan->algo = FSB_ALGO_MERGE;
-        plan->items_per_unit = kMergeThreads * (esz <= 4 ? 8 : 4);
+        plan->items_per_unit = spmv_merge_items(A);
         plan->n_units = ceil_div(A->n_rows + A->nnz, plan->items_per_unit);
         return;
     }
-    double v = A->n_rows ? 2.0 * mean / vec : 32.0;
-    if (v < 1.0) v = 1.0;
-    int lanes = 1 << (int)std::nearbyint(std::log2(v));
     plan->algo = FSB_ALGO_ROWS;
-    plan->lanes = lanes < 2 ? 2 : (lanes > 32 ? 32 : lanes);
+    plan->lanes = A->n_rows ? spmv_row_lanes(A->n_rows, mean, vec, skewed) : 32;
     plan->flags = FSB_PLAN_OVERLAP_LAUNCH;
 }
 
@@ -399,7 +538,7 @@ int64_t checked_merge_bytes(const fsb_csr* A, int acc_mode, int out_dtype) {
     fsb_plan mp;
     memset(&mp, 0, sizeof(mp));
     mp.algo = FSB_ALGO_MERGE;
-    mp.items_per_unit = kMergeThreads * (elem_size(A->value_dtype) <= 4 ? 8 : 4);
+    mp.items_per_unit = spmv_merge_items(A);
     mp.n_units = ceil_div(A->n_rows + A->nnz, mp.items_per_unit);
     const int64_t coords = align_up((mp.n_units + 1) * 2 * (int64_t)sizeof(int64_t), 256);
     return coords + fsb_workspace_bytes(0, A, 1, acc_mode, out_dtype, &mp);
@@ -612,9 +751,10 @@ extern "C" int fsb_spmv_csr_noalloc(const fsb_csr* A, const void* x, void* y, in
                 MergeScratch ms = merge_scratch_carve(carries, n_tiles, 1, (int)sizeof(Ac));
                 O* yv = static_cast<O*>(y);
                 const I* rmap = static_cast<const I*>(A->row_map);
-                k_spmv_merge<V, Ac, O, I, P><<<(unsigned)n_tiles, kMergeThreads, 0, st>>>(
+                k_spmv_merge<V, Ac, O, I, P><<<(unsigned)ceil_div(n_tiles, kMergeThreads / 32), kMergeThreads, 0, st>>>(
                     static_cast<const V*>(A->values), static_cast<const I*>(A->col_idx), ptr, rmap,
-                    static_cast<const V*>(x), yv, A->n_rows, coords, items_per_unit / kMergeThreads, ms.carry_row,
+                    static_cast<const V*>(x), yv, A->n_rows, A->nnz,
+                    aligned16(A->values) && aligned16(A->col_idx), coords, n_tiles, ms.carry_row,
                     static_cast<Ac*>(ms.carry_val), static_cast<Ac*>(ms.head_val));
                 rc2 = fsb_host::check_launch("k_spmv_merge (noalloc)");
                 if (rc2) return rc2;
