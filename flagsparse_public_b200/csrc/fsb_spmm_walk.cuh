@@ -36,7 +36,8 @@ constexpr int kWalkChunk = 256;
 // Resident CTAs of 128 threads per SM requested from the compiler.  For
 // accumulators of 16 bytes per lane, power law at N = 64: 5 CTAs (96
 // registers) 95 us, 6 (80) 81, 7 (72) 90, 8 (64, spills) 101; 4 CTAs with 16
-// loads in flight per lane 92.
+// loads in flight per lane 92.  32 bytes per lane (float64 sums, N = 64): 5 CTAs
+// 134, 4 CTAs 138 us at 256 items.
 template <class V, class A, int VW> struct WalkMinBlocks {
     static constexpr int acc_bytes = (int)sizeof(A) * VW;
     static constexpr int value = acc_bytes <= 16 ? 6 : (acc_bytes <= 32 ? 5 : 4);
@@ -310,21 +311,25 @@ k_spmm_walk(const V* __restrict__ val, const I* __restrict__ col, const void* __
 #pragma unroll
                         for (int u = 0; u < U; ++u) a[u] = u < cnt ? s_val[e + u] : vzero<V>();
                     }
-                    // a batch's products are summed on their own and enter the
-                    // row's sum once: chains of U + length / U additions
-                    A t[VW];
-                    zero_acc<A, VW>(t);
+                    // a batch's products are summed on their own, in two chains,
+                    // and enter the row's sum once
+                    A t[2][VW];
+                    zero_acc<A, VW>(t[0]);
+                    zero_acc<A, VW>(t[1]);
+                    auto join = [&]() {
+#pragma unroll
+                        for (int w = 0; w < VW; ++w) acc[w] = acc_add(acc[w], acc_add(t[0][w], t[1][w]));
+                    };
                     if (!__any_sync(full, bits != 0u)) {
 #pragma unroll
                         for (int u = 0; u < U; ++u)
 #pragma unroll
-                            for (int w = 0; w < VW; ++w) t[w] = Acc<V, A>::fma(a[u], bv[u].v[w], t[w]);
+                            for (int w = 0; w < VW; ++w) t[u & 1][w] = Acc<V, A>::fma(a[u], bv[u].v[w], t[u & 1][w]);
                     } else {
 #pragma unroll
                         for (int u = 0; u < U; ++u) {
                             if (bits & (1u << u)) {
-#pragma unroll
-                                for (int w = 0; w < VW; ++w) acc[w] = acc_add(acc[w], t[w]);
+                                join();
                                 if (cont) {
 #pragma unroll
                                     for (int w = 0; w < VW; ++w) sm_head[threadIdx.x][w] = acc[w];
@@ -334,14 +339,14 @@ k_spmm_walk(const V* __restrict__ val, const I* __restrict__ col, const void* __
                                 }
                                 rcur = s_row[e + u];
                                 zero_acc<A, VW>(acc);
-                                zero_acc<A, VW>(t);
+                                zero_acc<A, VW>(t[0]);
+                                zero_acc<A, VW>(t[1]);
                             }
 #pragma unroll
-                            for (int w = 0; w < VW; ++w) t[w] = Acc<V, A>::fma(a[u], bv[u].v[w], t[w]);
+                            for (int w = 0; w < VW; ++w) t[u & 1][w] = Acc<V, A>::fma(a[u], bv[u].v[w], t[u & 1][w]);
                         }
                     }
-#pragma unroll
-                    for (int w = 0; w < VW; ++w) acc[w] = acc_add(acc[w], t[w]);
+                    join();
                 };
                 for (int it = 0; it < base; ++it) batch(e_lo + it * U, U, true);
                 if (nb * U < n || extra > 0) batch(e_lo + base * U, ragged, false);

@@ -279,16 +279,34 @@ k_spmv_merge(const V* __restrict__ val, const I* __restrict__ col, const P* __re
         A acc = Acc<V, A>::zero(), head = Acc<V, A>::zero();
         int rcur = 0;
         bool broke = false;
+        uint32_t any_flag = fl[0];
+        if constexpr (E == 8) any_flag |= fl[1];
+        if (any_flag == 0u) {
+            // no row starts here: pairs, then their tree (a long row's sum
+            // rounds as often as if many lanes shared it)
+            A t[E / 2];
 #pragma unroll
-        for (int u = 0; u < E; ++u) {
-            if (fl[u / 4] & (1u << (8 * (u % 4)))) {
-                if (broke) put(rcur, acc);
-                else head = acc;
-                broke = true;
-                rcur = s_row[lane * E + u];
-                acc = Acc<V, A>::zero();
+            for (int i = 0; i < E / 2; ++i) t[i] = Acc<V, A>::zero();
+#pragma unroll
+            for (int u = 0; u < E; ++u)
+                if (whole || ((valid >> u) & 1u)) t[u / 2] = Acc<V, A>::fma(v[u], xv[u], t[u / 2]);
+#pragma unroll
+            for (int n = E / 2; n > 1; n /= 2)
+#pragma unroll
+                for (int i = 0; i < n / 2; ++i) t[i] = acc_add(t[2 * i], t[2 * i + 1]);
+            acc = t[0];
+        } else {
+#pragma unroll
+            for (int u = 0; u < E; ++u) {
+                if (fl[u / 4] & (1u << (8 * (u % 4)))) {
+                    if (broke) put(rcur, acc);
+                    else head = acc;
+                    broke = true;
+                    rcur = s_row[lane * E + u];
+                    acc = Acc<V, A>::zero();
+                }
+                if (whole || ((valid >> u) & 1u)) acc = Acc<V, A>::fma(v[u], xv[u], acc);
             }
-            if (whole || ((valid >> u) & 1u)) acc = Acc<V, A>::fma(v[u], xv[u], acc);
         }
         // lanes in order: the open row's sum enters at lane 0, each lane's tail
         // passes on to the lanes up to (and into) the next one holding a break
