@@ -9,15 +9,17 @@
 // Radix sort: 8-bit digits, least significant first, one pass per digit of
 // the caller's key width (key_bits).  A pass is three kernels over tiles of
 // kTile keys:
-//   * k_sort_upsweep: per-tile digit histogram (warp-aggregated shared-memory
-//     counts), stored digit-major: hist[digit][tile];
+//   * k_sort_upsweep: per-tile digit histogram (shared-memory atomics, all of a
+//     thread's keys loaded first), stored digit-major: hist[digit][tile];
 //   * k_scan_rows: one CTA per digit scans its row of tile counts in place
 //     (exclusive) and records the digit's total;
-//   * k_sort_downsweep: each tile scans the 256 totals for the digit starts,
-//     then ranks its keys in rounds of 256 (one per thread, in key order):
-//     __match_any_sync groups the warp's equal digits, per-warp digit counts
-//     in shared memory are prefixed over the warps by the thread that owns
-//     the digit; the tile is staged in shared memory in digit order and
+//   * k_sort_downsweep: each tile scans the 256 totals for the digit starts;
+//     each warp ranks its 512 consecutive keys on its own, 32 per round
+//     (__match_any_sync groups the equal digits, the warp's digit counts in
+//     shared memory); the counts are then prefixed over the warps once, by the
+//     thread that owns the digit (2.1 M 18-bit keys, three passes: 136 us with
+//     three CTA barriers per 256 keys and warp-aggregated histograms, 92
+//     like this).  The tile is staged in shared memory in digit order and
 //     written out in order, key and permutation entry to digit start + tile
 //     prefix + rank.  Ranks follow key order inside the tile and tiles
 //     follow each other, so every pass is stable and the result equals a
@@ -76,17 +78,18 @@ __global__ void __launch_bounds__(kThreads)
 k_sort_upsweep(const K* __restrict__ keys, int64_t n, K flip, int shift, uint32_t mask, uint32_t* __restrict__ hist,
                int64_t n_tiles) {
     __shared__ uint32_t h[kBins];
-    const int lane = threadIdx.x & 31;
     h[threadIdx.x] = 0u;
     __syncthreads();
     const int64_t t0 = (int64_t)blockIdx.x * kTile;
-#pragma unroll 4
+    K k[kRounds];
+#pragma unroll
     for (int r = 0; r < kRounds; ++r) {
         const int64_t i = t0 + (int64_t)r * kThreads + threadIdx.x;
-        const int d = i < n ? digit_of<K>(keys[i] ^ flip, shift, mask) : kBins;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        if (d < kBins && (peers & ((1u << lane) - 1u)) == 0u) atomicAdd(&h[d], (uint32_t)__popc(peers));
+        k[r] = i < n ? keys[i] : K(0);
     }
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r)
+        if (t0 + (int64_t)r * kThreads + threadIdx.x < n) atomicAdd(&h[digit_of<K>(k[r] ^ flip, shift, mask)], 1u);
     __syncthreads();
     hist[(int64_t)threadIdx.x * n_tiles + blockIdx.x] = h[threadIdx.x];
 }
@@ -131,7 +134,7 @@ k_sort_downsweep(const K* __restrict__ keys_in, K in_flip, const PIn* __restrict
                  const uint32_t* __restrict__ hist, const uint32_t* __restrict__ totals, int64_t n_tiles) {
     __shared__ uint32_t gbase[kBins];  // output position of the tile's first key of each digit
     __shared__ uint32_t lbase[kBins];  // its position in the staged tile
-    __shared__ uint32_t wcnt[2][kWarps][kBins];
+    __shared__ uint32_t wcnt[kWarps][kBins];  // per warp: its keys of each digit, then those of the warps before it
     __shared__ uint32_t sums[kWarps];
     extern __shared__ __align__(16) unsigned char staged[];  // downsweep_smem<K>() bytes
     K* skey = reinterpret_cast<K*>(staged);
@@ -139,11 +142,12 @@ k_sort_downsweep(const K* __restrict__ keys_in, K in_flip, const PIn* __restrict
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t t0 = (int64_t)blockIdx.x * kTile;
     const int n_here = (int)((n - t0) < kTile ? (n - t0) : kTile);
+    const int first = warp * (kRounds * 32) + lane;  // the warp's keys are consecutive
     K k[kRounds];
     uint32_t src[kRounds];
 #pragma unroll
     for (int r = 0; r < kRounds; ++r) {
-        const int64_t i = t0 + (int64_t)r * kThreads + tid;
+        const int64_t i = t0 + first + r * 32;
         k[r] = 0;
         src[r] = 0;
         if (i < n) {
@@ -151,37 +155,35 @@ k_sort_downsweep(const K* __restrict__ keys_in, K in_flip, const PIn* __restrict
             src[r] = perm_in ? (uint32_t)perm_in[i] : (uint32_t)i;
         }
     }
-    {
-        const uint32_t tot = totals[tid];
-        uint32_t all;
-        const uint32_t start = block_scan(tot, sums, &all) - tot;
-        gbase[tid] = start + hist[(int64_t)tid * n_tiles + blockIdx.x];
-    }
-    uint32_t run = 0;  // keys of digit tid ranked so far in this tile
+#pragma unroll
+    for (int i = 0; i < kBins / 32; ++i) wcnt[warp][i * 32 + lane] = 0u;
+    __syncwarp();
+    // ranks among the warp's keys of the same digit: no CTA barrier per round
     uint32_t rank[kRounds];
 #pragma unroll
     for (int r = 0; r < kRounds; ++r) {
-        uint32_t(*cnt)[kBins] = wcnt[r & 1];
-        const bool ok = r * kThreads + tid < n_here;
+        const bool ok = first + r * 32 < n_here;
         const int d = ok ? digit_of<K>(k[r], shift, mask) : kBins;  // lanes past the end: no real digit
         const unsigned peers = __match_any_sync(0xffffffffu, d);
         const uint32_t lrank = (uint32_t)__popc(peers & ((1u << lane) - 1u));
+        const uint32_t before = ok ? wcnt[warp][d] : 0u;
+        __syncwarp();
+        if (ok && lrank == 0u) wcnt[warp][d] = before + (uint32_t)__popc(peers);
+        __syncwarp();
+        rank[r] = before + lrank;
+    }
+    {
+        const uint32_t tot = totals[tid];
+        uint32_t all;
+        const uint32_t start = block_scan(tot, sums, &all) - tot;  // (barriers: every warp has counted)
+        gbase[tid] = start + hist[(int64_t)tid * n_tiles + blockIdx.x];
+    }
+    uint32_t run = 0;  // the owner of digit tid: exclusive prefix over the warps
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) cnt[w][tid] = 0u;
-        __syncthreads();
-        if (ok && lrank == 0u) cnt[warp][d] = (uint32_t)__popc(peers);
-        __syncthreads();
-        // the owner of digit tid: exclusive prefix over the warps for these 256 keys
-        uint32_t acc = run;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const uint32_t c = cnt[w][tid];
-            cnt[w][tid] = acc;
-            acc += c;
-        }
-        run = acc;
-        __syncthreads();
-        rank[r] = ok ? cnt[warp][d] + lrank : 0u;
+    for (int w = 0; w < kWarps; ++w) {
+        const uint32_t c = wcnt[w][tid];
+        wcnt[w][tid] = run;
+        run += c;
     }
     {
         uint32_t all;
@@ -190,8 +192,9 @@ k_sort_downsweep(const K* __restrict__ keys_in, K in_flip, const PIn* __restrict
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < kRounds; ++r) {
-        if (r * kThreads + tid < n_here) {
-            const uint32_t p = lbase[digit_of<K>(k[r], shift, mask)] + rank[r];
+        if (first + r * 32 < n_here) {
+            const int d = digit_of<K>(k[r], shift, mask);
+            const uint32_t p = lbase[d] + wcnt[warp][d] + rank[r];
             skey[p] = k[r];
             sidx[p] = src[r];
         }
@@ -368,8 +371,11 @@ int run_sort(const K* keys, int64_t n, int key_bits, bool signed_full, K* keys_o
     uint32_t* pb[2] = {reinterpret_cast<uint32_t*>(ws + L.perm_a), reinterpret_cast<uint32_t*>(ws + L.perm_b)};
     const unsigned grid = (unsigned)L.n_tiles;
     for (int p = 0; p < L.passes; ++p) {
-        const int shift = 8 * p;
-        const int bits = key_bits - shift < 8 ? key_bits - shift : 8;
+        // even digits: 18 bits go 6 + 6 + 6, not 8 + 8 + 2 -- a tile's runs of
+        // equal digits are then four times as long where it is written out
+        const int per = (key_bits + (int)L.passes - 1) / (int)L.passes;
+        const int shift = per * p;
+        const int bits = key_bits - shift < per ? key_bits - shift : per;
         const uint32_t mask = (1u << bits) - 1u;
         const bool first = p == 0, last = p == L.passes - 1;
         const K* kin = first ? keys : kb[(p - 1) & 1];
