@@ -212,6 +212,17 @@ _SIGNATURES = {
          ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p,
          ctypes.c_int64, ctypes.c_int, ctypes.c_void_p],
     ),
+    "fsb_coo_check_workspace_bytes": (ctypes.c_int64, [ctypes.c_int64]),
+    "fsb_coo_check": (
+        ctypes.c_int,
+        [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_void_p,
+         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p],
+    ),
+    "fsb_take_entries": (
+        ctypes.c_int,
+        [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p,
+         ctypes.c_void_p, ctypes.c_void_p],
+    ),
     "fsb_sorted_keys_to_offsets": (
         ctypes.c_int,
         [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p],
@@ -344,15 +355,40 @@ def ptr(t):
 _figures = threading.local()
 
 
+def _figure_buffer():
+    """This thread's pinned buffer of eight figures."""
+    buf = getattr(_figures, "buf", None)
+    if buf is None:
+        buf = _figures.buf = torch.empty(8, dtype=torch.int64).pin_memory()
+    return buf
+
+
+def coo_check(row, col):
+    """((min row, max row, min col, max col), row as int32, col as int32) of
+    contiguous COO indices with at least one entry: fsb_coo_check, read after
+    one stream synchronisation.  int32 inputs come back as they are; wider
+    ones truncated, so the caller looks at the figures first."""
+    buf = _figure_buffer()
+    nnz, dev = int(row.numel()), row.device
+    lib = library()
+    row32 = torch.empty(nnz, dtype=torch.int32, device=dev) if row.dtype != torch.int32 else None
+    col32 = torch.empty(nnz, dtype=torch.int32, device=dev) if col.dtype != torch.int32 else None
+    nbytes = int(lib.fsb_coo_check_workspace_bytes(nnz))
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    rc = lib.fsb_coo_check(ptr(row), dtype_code(row.dtype), ptr(col), dtype_code(col.dtype), nnz, ptr(row32),
+                           ptr(col32), ctypes.c_void_p(buf.data_ptr()), ptr(ws), nbytes, stream_handle(dev))
+    check(rc, "fsb_coo_check")
+    torch.cuda.current_stream(dev).synchronize()
+    return buf.tolist()[:4], row if row32 is None else row32, col if col32 is None else col32
+
+
 def csr_check(row_ptr, col_idx, n_rows):
     """The eight structural figures of fsb_csr_check (row_ptr[0],
     row_ptr[n_rows], rows of negative length, negative column indices, largest
     column index, longest row, sum of squared row lengths, empty rows),
     written by its kernels into a pinned buffer of this thread and read after
     one stream synchronisation."""
-    buf = getattr(_figures, "buf", None)
-    if buf is None:
-        buf = _figures.buf = torch.empty(8, dtype=torch.int64).pin_memory()
+    buf = _figure_buffer()
     n_rows, nnz = int(n_rows), int(col_idx.numel())
     lib = library()
     nbytes = int(lib.fsb_csr_check_workspace_bytes(n_rows, nnz))

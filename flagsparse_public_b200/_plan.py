@@ -181,6 +181,16 @@ class KernelPlan:
                              runs=self.runs if finish else None, tickets=self.tickets if finish else None)
 
 
+def one_shot(plan):
+    """``plan`` for a single product: split rows finish in the fix-up kernel
+    rather than by tickets, which need the unit runs, zeroed counters and a
+    host read first (about 30 us of launches and waiting; the fix-up launch
+    costs 5)."""
+    if isinstance(plan, KernelPlan) and plan._seq_registers():
+        plan.runs = False
+    return plan
+
+
 # Plan kind (host side only) of the tensor-core BSR candidate.
 ALGO_BSR = -1
 # Largest fill-in the BSR candidate accepts: stored block entries (256 per
@@ -453,6 +463,19 @@ def stable_sort(keys, key_bound=None):
                              nat.stream_handle(keys.device))
     nat.check(rc, "fsb_stable_sort")
     return out, order
+
+
+def take_entries(values, col, order):
+    """(values[order], col[order]) of COO entries on the device with int32
+    columns (fsb_take_entries: one pass over the permutation)."""
+    values, col = values.contiguous(), col.contiguous()
+    n = order.numel()
+    out_v = torch.empty(n, dtype=values.dtype, device=values.device)
+    out_c = torch.empty(n, dtype=col.dtype, device=col.device)
+    rc = nat.library().fsb_take_entries(nat.ptr(order), n, nat.ptr(values), values.element_size(), nat.ptr(out_v),
+                                        nat.ptr(col), nat.ptr(out_c), nat.stream_handle(values.device))
+    nat.check(rc, "fsb_take_entries")
+    return out_v, out_c
 
 
 def run_starts_device(sorted_keys, out_dtype):

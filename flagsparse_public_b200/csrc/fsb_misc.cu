@@ -136,6 +136,96 @@ __global__ void __launch_bounds__(kCheckThreads) k_csr_check_final(const P* __re
     }
 }
 
+// Smallest and largest row and column of COO entries, and the indices
+// narrowed to 32 bits where asked for, in one read of both arrays: FlagSparse's
+// four reductions (spmm_coo.py:325-343) and its two int32 conversions.
+constexpr int kCooThreads = 256;
+constexpr int kCooMaxBlocks = 148 * 4;
+
+__device__ __forceinline__ void coo_fold(int64_t (&v)[4], const int64_t (&o)[4]) {
+    v[0] = o[0] < v[0] ? o[0] : v[0];
+    v[1] = o[1] > v[1] ? o[1] : v[1];
+    v[2] = o[2] < v[2] ? o[2] : v[2];
+    v[3] = o[3] > v[3] ? o[3] : v[3];
+}
+
+// Result in v of thread 0.
+__device__ __forceinline__ void coo_block_fold(int64_t (&v)[4]) {
+    __shared__ int64_t red[kCooThreads / 32][4];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        int64_t t[4];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) t[f] = __shfl_xor_sync(0xffffffffu, v[f], o);
+        coo_fold(v, t);
+    }
+    const int warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) red[warp][f] = v[f];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kCooThreads / 32; ++w) coo_fold(v, red[w]);
+    }
+}
+
+template <class R, class K>
+__global__ void __launch_bounds__(kCooThreads) k_coo_check_part(const R* __restrict__ row, const K* __restrict__ col,
+                                                                int64_t nnz, int32_t* __restrict__ row32,
+                                                                int32_t* __restrict__ col32,
+                                                                int64_t* __restrict__ part) {
+    int64_t v[4] = {INT64_MAX, INT64_MIN, INT64_MAX, INT64_MIN};
+    const int64_t stride = (int64_t)gridDim.x * kCooThreads;
+#pragma unroll 4
+    for (int64_t k = (int64_t)blockIdx.x * kCooThreads + threadIdx.x; k < nnz; k += stride) {
+        const int64_t r = idx(row[k]), c = idx(col[k]);
+        const int64_t t[4] = {r, r, c, c};
+        coo_fold(v, t);
+        if (row32) row32[k] = (int32_t)r;
+        if (col32) col32[k] = (int32_t)c;
+    }
+    coo_block_fold(v);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) part[(int64_t)blockIdx.x * 4 + f] = v[f];
+    }
+}
+
+__global__ void __launch_bounds__(kCooThreads) k_coo_check_final(const int64_t* __restrict__ part, int n_parts,
+                                                                 int64_t* out) {
+    int64_t v[4] = {INT64_MAX, INT64_MIN, INT64_MAX, INT64_MIN};
+    for (int b = threadIdx.x; b < n_parts; b += kCooThreads) {
+        const int64_t t[4] = {part[4 * b], part[4 * b + 1], part[4 * b + 2], part[4 * b + 3]};
+        coo_fold(v, t);
+    }
+    coo_block_fold(v);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) out[f] = v[f];
+    }
+}
+
+// values[order] and col[order] in one pass over the permutation (element
+// copies; T is a carrier of the values' size).
+template <class T>
+__global__ void __launch_bounds__(256) k_take_entries(const int64_t* __restrict__ order, int64_t n,
+                                                      const T* __restrict__ values, T* __restrict__ values_out,
+                                                      const int32_t* __restrict__ col, int32_t* __restrict__ col_out) {
+    const int64_t stride = (int64_t)gridDim.x * 256;
+#pragma unroll 4
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += stride) {
+        const int64_t k = order[i];
+        values_out[i] = values[k];
+        col_out[i] = col[k];
+    }
+}
+
+static int64_t coo_check_blocks(int64_t nnz) {
+    const int64_t b = ceil_div(nnz, (int64_t)kCooThreads * 8);
+    return b < 1 ? 1 : (b > kCooMaxBlocks ? kCooMaxBlocks : b);
+}
+
 static int64_t check_blocks(int64_t n_rows, int64_t nnz) {
     const int64_t work = n_rows > nnz ? n_rows : nnz;
     const int64_t b = ceil_div(work, (int64_t)kCheckThreads * 8);
@@ -244,6 +334,70 @@ extern "C" int fsb_csr_check(const void* row_ptr, int ptr_dtype, int64_t n_rows,
                                                           (int)blocks, out);
         return fsb_host::check_launch("k_csr_check_final");
     });
+}
+
+extern "C" int64_t fsb_coo_check_workspace_bytes(int64_t nnz) {
+    return nnz < 0 ? 0 : coo_check_blocks(nnz) * 4 * (int64_t)sizeof(int64_t);
+}
+
+extern "C" int fsb_coo_check(const void* row, int row_dtype, const void* col, int col_dtype, int64_t nnz,
+                             int32_t* row32, int32_t* col32, int64_t* out, void* workspace, int64_t workspace_bytes,
+                             void* stream) {
+    if (nnz < 1 || !row || !col || !out) {
+        fsb_host::set_error("fsb_coo_check: no entries or a null pointer");
+        return FSB_ERR_INVALID;
+    }
+    if (!workspace || workspace_bytes < fsb_coo_check_workspace_bytes(nnz)) {
+        fsb_host::set_error("fsb_coo_check: workspace %lld bytes < %lld", (long long)workspace_bytes,
+                            (long long)fsb_coo_check_workspace_bytes(nnz));
+        return FSB_ERR_WORKSPACE;
+    }
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    int64_t* part = static_cast<int64_t*>(workspace);
+    const int64_t blocks = coo_check_blocks(nnz);
+    return dispatch_idx(row_dtype, [&](auto tr) -> int {
+        using R = typename decltype(tr)::type;
+        return dispatch_idx(col_dtype, [&](auto tc) -> int {
+            using K = typename decltype(tc)::type;
+            k_coo_check_part<R, K><<<(unsigned)blocks, kCooThreads, 0, st>>>(
+                static_cast<const R*>(row), static_cast<const K*>(col), nnz, row32, col32, part);
+            const int rc = fsb_host::check_launch("k_coo_check_part");
+            if (rc) return rc;
+            k_coo_check_final<<<1, kCooThreads, 0, st>>>(part, (int)blocks, out);
+            return fsb_host::check_launch("k_coo_check_final");
+        });
+    });
+}
+
+extern "C" int fsb_take_entries(const int64_t* order, int64_t n, const void* values, int value_bytes, void* values_out,
+                                const int32_t* col, int32_t* col_out, void* stream) {
+    if (n < 0) {
+        fsb_host::set_error("fsb_take_entries: negative size");
+        return FSB_ERR_INVALID;
+    }
+    if (n == 0) return FSB_OK;
+    if (!order || !values || !values_out || !col || !col_out) {
+        fsb_host::set_error("fsb_take_entries: null pointer");
+        return FSB_ERR_INVALID;
+    }
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int64_t want = ceil_div(n, (int64_t)256 * 4);
+    const unsigned grid = (unsigned)(want > 148 * 32 ? 148 * 32 : want);
+    auto go = [&](auto t) -> int {
+        using T = typename decltype(t)::type;
+        k_take_entries<T><<<grid, 256, 0, st>>>(order, n, static_cast<const T*>(values), static_cast<T*>(values_out),
+                                                col, col_out);
+        return fsb_host::check_launch("k_take_entries");
+    };
+    switch (value_bytes) {
+    case 2: return go(tag<raw_type<2>::T>{});
+    case 4: return go(tag<raw_type<4>::T>{});
+    case 8: return go(tag<raw_type<8>::T>{});
+    case 16: return go(tag<raw_type<16>::T>{});
+    default:
+        fsb_host::set_error("fsb_take_entries: values of %d bytes", value_bytes);
+        return FSB_ERR_UNSUPPORTED;
+    }
 }
 
 // Value/accumulator pairs of the atomic routes: the accumulator buffer is the

@@ -117,10 +117,13 @@ def _prepare_spmm_coo_inputs(data, row, col, B, shape):
         raise ValueError("nnz exceeds the int32 range supported by the Triton COO kernel")
     # the index checks read the device: skipped while a CUDA graph records
     # the call (the caller checks the indices before capturing)
+    data = data.contiguous()
+    row = row.contiguous()
+    col = col.contiguous()
+    kernel_row = kernel_col = None
     if nnz > 0 and not torch.cuda.is_current_stream_capturing():
-        lim = torch.stack([row.min().to(torch.int64), row.max().to(torch.int64), col.min().to(torch.int64),
-                           col.max().to(torch.int64)]).tolist()
-        min_row, max_row, min_col, max_col = lim
+        # the four bounds and the int32 indices in one read of both arrays
+        (min_row, max_row, min_col, max_col), kernel_row, kernel_col = _nat.coo_check(row, col)
         if min_row < 0 or max_row >= n_rows:
             raise IndexError("row indices out of range for n_rows")
         if min_col < 0 or max_col >= n_cols:
@@ -129,12 +132,10 @@ def _prepare_spmm_coo_inputs(data, row, col, B, shape):
             raise ValueError("row indices exceed the int32 range supported by the Triton kernel")
         if max_col > _INDEX_LIMIT_INT32:
             raise ValueError("column indices exceed the int32 range supported by the Triton kernel")
-    data = data.contiguous()
-    row = row.contiguous()
-    col = col.contiguous()
     B = B.contiguous()
-    kernel_row = row.to(torch.int32) if row.dtype == torch.int64 else row
-    kernel_col = col.to(torch.int32) if col.dtype == torch.int64 else col
+    if kernel_row is None:
+        kernel_row = row.to(torch.int32) if row.dtype == torch.int64 else row
+        kernel_col = col.to(torch.int32) if col.dtype == torch.int64 else col
     return data, kernel_row, kernel_col, B, n_rows, n_cols, int(B.shape[1])
 
 
@@ -174,12 +175,15 @@ def _take(values, order):
 
 
 def _coo_rows_to_csr(data, row, col, n_rows):
-    """Order nonzeros by row (stable) and build int64 row offsets."""
-    row64 = row.to(torch.int64)
+    """Order nonzeros by row (stable) and build int64 row offsets.  int32 rows
+    are sorted as they are (half the key bytes of an int64 sort per pass)."""
     if data.numel() > 1:
-        sorted_rows, order = _plan.stable_sort(row64, key_bound=n_rows)
-        data, col, row64 = _take(data, order), col[order], sorted_rows
-    indptr = _plan.sorted_keys_to_offsets(row64, n_rows)
+        row, order = _plan.stable_sort(row, key_bound=n_rows)
+        if data.is_cuda and col.dtype == torch.int32:
+            data, col = _plan.take_entries(data, col, order)
+        else:
+            data, col = _take(data, order), col[order]
+    indptr = _plan.sorted_keys_to_offsets(row, n_rows)
     return data.contiguous(), col.contiguous(), indptr
 
 
@@ -200,7 +204,7 @@ def _triton_spmm_coo_impl(data, row, col, B, n_rows, n_dense_cols, block_n, bloc
         # nonzeros per unit): no statistics read from the device
         nnz = data.numel()
         stats = _plan.MatrixStats(n_rows, B.shape[0], nnz, nnz, nnz / max(n_rows, 1), 0.0, 0)
-        plan = _plan.default_spmm_plan(stats, n_dense_cols, data.dtype)
+        plan = _plan.one_shot(_plan.default_spmm_plan(stats, n_dense_cols, data.dtype))
         _plan.run_spmm(d, c, indptr, n_rows, B.shape[0], B, C, _acc_mode_for(data.dtype), plan)
         return C if C.dtype == out_dtype else C.to(out_dtype)
     acc_dtype = _spmm_coo_compute_dtype(data.dtype)

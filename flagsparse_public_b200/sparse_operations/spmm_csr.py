@@ -98,11 +98,13 @@ def _spmm_validation_metrics(candidate, reference):
     return metrics
 
 
-def _prepare_spmm_csr_matrix(data, indices, indptr, shape, return_stats=False):
+def _prepare_spmm_csr_matrix(data, indices, indptr, shape, return_stats=False, want_lengths=True):
     """Validation of FlagSparse ``spmm_csr.py:197-255`` with one kernel and
     one device->host read for all structural checks.  Returns int32 column indices (int64 ones
     converted, as the reference does) and int64 indptr; with ``return_stats``
-    also the row-length statistics of the plan heuristics, from the same read."""
+    also the row-length statistics of the plan heuristics, from the same read.
+    ``want_lengths=False`` leaves the row lengths (used by prepared objects
+    only) out: None in their place."""
     if len(shape) != 2:
         raise ValueError("shape must be a 2-tuple: (n_rows, n_cols)")
     if data.ndim != 1 or indices.ndim != 1 or indptr.ndim != 1:
@@ -142,7 +144,7 @@ def _prepare_spmm_csr_matrix(data, indices, indptr, shape, return_stats=False):
             raise IndexError("indices out of range for n_cols")
         if c[4] > _INDEX_LIMIT_INT32:
             raise ValueError("column indices exceed the int32 range supported by the Triton kernel")
-    row_lengths = (indptr[1:] - indptr[:-1]).to(torch.int64)
+    row_lengths = (indptr[1:] - indptr[:-1]).to(torch.int64) if want_lengths else None
     kernel_indices = indices.to(torch.int32) if indices.dtype == torch.int64 else indices
     kernel_indptr = indptr.to(torch.int64)
     max_row_nnz = c[5]
@@ -162,7 +164,7 @@ def _prepare_spmm_csr_inputs(data, indices, indptr, B, shape):
     if B.ndim != 2:
         raise ValueError("B must be a 2D dense tensor")
     data, kernel_indices, kernel_indptr, n_rows, n_cols, _rl, max_row_nnz = _prepare_spmm_csr_matrix(
-        data, indices, indptr, shape
+        data, indices, indptr, shape, want_lengths=False
     )
     if B.shape[0] != n_cols:
         raise ValueError(f"B.shape[0] must be n_cols={n_cols}, got {B.shape[0]}")
@@ -242,6 +244,7 @@ class PreparedCsrSpmmOpt:
         "_bucket_meta",
         "_stats",
         "_plans",
+        "_one_shot",
     )
 
     def __init__(
@@ -279,6 +282,7 @@ class PreparedCsrSpmmOpt:
         self.long_row_fallback_only = bool(long_row_fallback_only)
         self._stats = None
         self._plans = {}
+        self._one_shot = False
 
     def _meta(self):
         if self._bucket_meta is None:
@@ -398,7 +402,12 @@ def _spmm_plan_for(holder, kind, n_dense, operands=None):
     if plan is None:
         if holder._stats is None:
             holder._stats = _plan.matrix_stats(holder.kernel_indptr, holder.n_rows, holder.n_cols)
-        if operands is not None and getattr(holder, "kernel_indices", None) is not None:
+        if getattr(holder, "_one_shot", False) and _plan.plan_selector() == "learned":
+            # a matrix multiplied once: the selector's feature pass, its two
+            # host reads and the split rows' ticket set-up cost more than the
+            # best plan saves on one product
+            plan = _plan.one_shot(_plan.default_spmm_plan(holder._stats, n_dense, holder.data.dtype))
+        elif operands is not None and getattr(holder, "kernel_indices", None) is not None:
             B, C, acc = operands
             plan = _plan.chosen_spmm_plan(holder._stats, holder.data, holder.kernel_indices, holder.kernel_indptr,
                                           holder.n_rows, holder.n_cols, B, C, acc)
@@ -444,7 +453,7 @@ def _triton_spmm_csr_impl(data, indices, indptr, B, n_rows, n_dense_cols, block_
         if max_row_nnz is None:
             max_row_nnz = int((indptr[1:] - indptr[:-1]).max().item())
         holder = _Alg1Holder(data, indptr, n_rows, B.shape[0], max_row_nnz, data.numel())
-        plan = _spmm_plan_for(holder, "alg1", n_dense_cols)
+        plan = _plan.one_shot(_spmm_plan_for(holder, "alg1", n_dense_cols))
     _plan.run_spmm(data, indices, indptr, n_rows, B.shape[0], B, C, _alg1_acc_mode(dtype), plan)
     return C
 
@@ -598,6 +607,7 @@ def flagsparse_spmm_csr_opt(data=None, indices=None, indptr=None, B=None, shape=
         if any(arg is None for arg in (data, indices, indptr, shape)):
             raise ValueError("data, indices, indptr, and shape are required when prepared is not provided")
         prepared = prepare_spmm_csr_opt(data, indices, indptr, shape)
+        prepared._one_shot = True  # this object does not outlive the call
     elif shape is not None:
         resolved_shape = (int(shape[0]), int(shape[1]))
         if resolved_shape != prepared.shape:

@@ -284,6 +284,22 @@ int fsb_spmm_coo_atomic(const void* values, const void* row, const void* col,
                         const void* B, int64_t ldb, int64_t n_dense, void* C,
                         int64_t ldc, int acc_dtype, void* stream);
 
+/* Smallest / largest row and column of nnz >= 1 COO entries, out[4] = {min
+ * row, max row, min col, max col} (device or pinned host memory, written by
+ * the kernels on the stream), and, where row32 / col32 are not null, the
+ * indices narrowed to 32 bits.  One read of both arrays; replaces the four
+ * reductions and two conversions of _prepare_spmm_coo_inputs
+ * (spmm_coo.py:54-118).  workspace: fsb_coo_check_workspace_bytes(nnz).    */
+int64_t fsb_coo_check_workspace_bytes(int64_t nnz);
+int fsb_coo_check(const void* row, int row_dtype, const void* col, int col_dtype,
+                  int64_t nnz, int32_t* row32, int32_t* col32, int64_t* out,
+                  void* workspace, int64_t workspace_bytes, void* stream);
+
+/* values_out[i] = values[order[i]], col_out[i] = col[order[i]] for values of
+ * value_bytes (2, 4, 8 or 16) each: the entries of a sorted COO matrix.    */
+int fsb_take_entries(const int64_t* order, int64_t n, const void* values, int value_bytes,
+                     void* values_out, const int32_t* col, int32_t* col_out, void* stream);
+
 /* offsets[b] = number of keys below b for b = 0 .. n_bins (n_bins + 1
  * entries) from nondecreasing keys in [0, n_bins): CSR row offsets of sorted
  * COO rows, column offsets of a transpose.  No host synchronisation (can be
