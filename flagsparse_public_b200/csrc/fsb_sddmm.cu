@@ -3,72 +3,122 @@
 // for every stored position p (FlagSparse's flagsparse_sddmm_csr,
 // sddmm_csr.py:350-422, kernel _sddmm_csr_real_kernel :108-152).
 //
-// A sub-group of LPN lanes computes one dot product, each lane covering VW
-// consecutive elements of K per step (16-byte vectors where x and y allow);
-// a warp takes NPAR = 32 / LPN positions per step and kSddmmU steps per
-// batch, whose x / y loads are all issued before the multiply-adds use them
-// (the y rows are random gathers, latency bound).  The dot product is reduced
-// inside its sub-group (log2 LPN xor-shuffles).  float32 accumulates in
-// float32, float64 in float64, as FlagSparse's baseline kernel does.
+// A sub-group of LPN lanes computes kSddmmU consecutive positions at a time,
+// each lane covering VW consecutive elements of K per step (16-byte vectors
+// where x and y allow).  The positions' indices come as vector loads, their y
+// rows are loaded back to back (random gathers, latency bound), and x is
+// loaded once where the positions of every sub-group lie in one row each.  The
+// dot products are reduced together: each halving step exchanges half of the
+// sums (5 shuffles for 4 products over 16 lanes where one reduction each took
+// 16), and the lanes that end with them store neighbouring results.
+// float32 accumulates in float32, float64 in float64, as FlagSparse's baseline
+// kernel does.
 #include "fsb_dispatch.cuh"
 
 namespace fsb {
 
 constexpr int kSddmmThreads = 256;
-constexpr int kSddmmU = 4;
+constexpr int kSddmmU = 4;  // positions per sub-group and batch
 
-// 4 resident CTAs of 256 threads per SM (64 registers): the random y-row
-// gathers are latency bound, so resident warps beat unspilled registers
-// (measured: 80 registers / 3 CTAs 0.239 ms, 64 / 4 0.188 ms, 51 / 5
-// 0.197 ms on the power-law pattern at K = 64).
+// The indices of a batch from position p0 on (clamped to the last of n; 16-byte loads
+// where they are aligned and all inside).
+template <class I>
+__device__ __forceinline__ void load_indices(const I* __restrict__ a, int64_t p0, int64_t n, bool vec_ok,
+                                             I (&out)[kSddmmU]) {
+    if (vec_ok && p0 + kSddmmU <= n) {
+        constexpr int M = 16 / (int)sizeof(I) < kSddmmU ? 16 / (int)sizeof(I) : kSddmmU;
+#pragma unroll
+        for (int i = 0; i < kSddmmU; i += M) {
+            const vec_t<I, M> t = ld_stream<I, M>(a + p0 + i);
+#pragma unroll
+            for (int j = 0; j < M; ++j) out[i + j] = t.v[j];
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < kSddmmU; ++u) out[u] = a[p0 + u < n ? p0 + u : n - 1];
+    }
+}
+
+// What bounds it: y rows in flight per SM.  Power-law pattern, 3.1 M
+// positions, before (a reduction per position, x loaded per position) -> now:
+// float32 K = 64 144 -> 130 us (its gathers alone: 68), K = 128 299 -> 251, K =
+// 143 (single elements) 598 -> 482, K = 200 754 -> 497; float64 K = 64 434 ->
+// 281.  Eight positions per batch: 151 us at 2 CTAs (128 registers), 186 at 3
+// (spills); 3 or 5 CTAs with four: 166 and 136.
 template <class V, class A, class I, int VW, int LPN_LOG2>
 __global__ void __launch_bounds__(kSddmmThreads, 4)
 k_sddmm(const I* __restrict__ col, const int32_t* __restrict__ row_ids, int64_t nnz, const V* __restrict__ x,
         int64_t ldx, const V* __restrict__ y, int64_t ldy, int64_t k, const V* __restrict__ data,
-        V* __restrict__ out, A alpha, A beta) {
+        V* __restrict__ out, A alpha, A beta, int vec_ok) {
     constexpr int LPN = 1 << LPN_LOG2;
     constexpr int NPAR = 32 >> LPN_LOG2;
-    constexpr int STEP = NPAR * kSddmmU;  // positions per warp batch
+    constexpr int U = kSddmmU;
+    constexpr int HALVINGS = LPN_LOG2 < 2 ? LPN_LOG2 : 2;  // log2 U at most
+    constexpr int LEFT = U >> HALVINGS;  // results per storing lane
+    constexpr unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int sub = lane >> LPN_LOG2, cl = lane & (LPN - 1);
     const int64_t warp = ((int64_t)blockIdx.x * kSddmmThreads + threadIdx.x) >> 5;
     const int64_t n_warps = ((int64_t)gridDim.x * kSddmmThreads) >> 5;
-    for (int64_t base = warp * STEP; base < nnz; base += n_warps * STEP) {
-        int64_t p[kSddmmU], r[kSddmmU], c[kSddmmU];
-        A acc[kSddmmU];
+    for (int64_t base = warp * (NPAR * U); base < nnz; base += n_warps * (NPAR * U)) {
+        const int64_t p0 = base + sub * U;
+        I c[U];
+        int32_t r[U];
+        load_indices<I>(col, p0, nnz, vec_ok, c);
+        load_indices<int32_t>(row_ids, p0, nnz, vec_ok, r);
+        bool same = true;
 #pragma unroll
-        for (int u = 0; u < kSddmmU; ++u) {
-            p[u] = base + u * NPAR + sub;
-            const bool ok = p[u] < nnz;
-            r[u] = ok ? (int64_t)row_ids[p[u]] : 0;
-            c[u] = ok ? idx(col[p[u]]) : 0;
-            acc[u] = A(0);
-        }
+        for (int u = 1; u < U; ++u) same = same && r[u] == r[0];
+        const bool one_row = __all_sync(full, same);
+        A acc[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc[u] = A(0);
         for (int64_t kk = (int64_t)cl * VW; kk < k; kk += (int64_t)LPN * VW) {
-            vec_t<V, VW> xv[kSddmmU], yv[kSddmmU];
+            vec_t<V, VW> yv[U];
 #pragma unroll
-            for (int u = 0; u < kSddmmU; ++u) {
-                if (p[u] < nnz) {
-                    xv[u] = ld_ro<V, VW>(x + r[u] * ldx + kk);
-                    yv[u] = ld_ro<V, VW>(y + c[u] * ldy + kk);
-                } else {
+            for (int u = 0; u < U; ++u) yv[u] = ld_ro<V, VW>(y + idx(c[u]) * ldy + kk);
+            if (one_row) {
+                const vec_t<V, VW> xv = ld_ro<V, VW>(x + (int64_t)r[0] * ldx + kk);
 #pragma unroll
-                    for (int w = 0; w < VW; ++w) xv[u].v[w] = yv[u].v[w] = V(0);
-                }
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int w = 0; w < VW; ++w) acc[u] = fma((A)xv.v[w], (A)yv[u].v[w], acc[u]);
+            } else {
+                vec_t<V, VW> xv[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) xv[u] = ld_ro<V, VW>(x + (int64_t)r[u] * ldx + kk);
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int w = 0; w < VW; ++w) acc[u] = fma((A)xv[u].v[w], (A)yv[u].v[w], acc[u]);
             }
+        }
+        // halving steps: the upper half of the lanes keeps the upper half of
+        // the sums, the lower half the lower
+        int first = 0;
 #pragma unroll
-            for (int u = 0; u < kSddmmU; ++u)
+        for (int h = 0; h < HALVINGS; ++h) {
+            const int o = LPN >> (h + 1), n = U >> (h + 1);
+            const bool upper = (cl & o) != 0;
 #pragma unroll
-                for (int w = 0; w < VW; ++w) acc[u] = fma((A)xv[u].v[w], (A)yv[u].v[w], acc[u]);
+            for (int i = 0; i < n; ++i) {
+                const A send = upper ? acc[i] : acc[i + n];
+                const A keep = upper ? acc[i + n] : acc[i];
+                acc[i] = keep + __shfl_xor_sync(full, send, o);
+            }
+            if (upper) first += n;
         }
 #pragma unroll
-        for (int u = 0; u < kSddmmU; ++u) {
+        for (int o = LPN >> (HALVINGS + 1); o > 0; o >>= 1) acc[0] += __shfl_xor_sync(full, acc[0], o);
+        if ((cl & ((LPN >> HALVINGS) - 1)) == 0) {
 #pragma unroll
-            for (int o = LPN / 2; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o, LPN);
-            if (cl == 0 && p[u] < nnz) {
-                A v = alpha * acc[u];
-                if (data) v += (A)data[p[u]] * beta;
-                out[p[u]] = (V)v;
+            for (int i = 0; i < LEFT; ++i) {
+                const int64_t p = p0 + first + i;
+                if (p < nnz) {
+                    A v = alpha * acc[i];
+                    if (data) v += (A)data[p] * beta;
+                    out[p] = (V)v;
+                }
             }
         }
     }
@@ -78,13 +128,14 @@ template <class V, class A, class I, int VW>
 int launch_sddmm_vw(int lpn_log2, const I* col, const int32_t* rows, int64_t nnz, const V* x, int64_t ldx, const V* y,
                     int64_t ldy, int64_t k, const V* data, V* out, A alpha, A beta, cudaStream_t st) {
     const int npar = 32 >> lpn_log2;
+    const int vec_ok = aligned16(col) && aligned16(rows);
     const int64_t warps = ceil_div(nnz, (int64_t)npar * kSddmmU);
     int64_t blocks = ceil_div(warps, (int64_t)(kSddmmThreads / 32));
     if (blocks > 148 * 64) blocks = 148 * 64;  // grid-stride beyond ~64 waves of CTAs
 #define FSB_SDDMM(L)                                                                                           \
     case L:                                                                                                    \
         k_sddmm<V, A, I, VW, L><<<(unsigned)blocks, kSddmmThreads, 0, st>>>(col, rows, nnz, x, ldx, y, ldy, k, \
-                                                                             data, out, alpha, beta);          \
+                                                                             data, out, alpha, beta, vec_ok);  \
         break;
     switch (lpn_log2) {
         FSB_SDDMM(0)
