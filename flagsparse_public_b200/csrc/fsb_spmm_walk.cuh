@@ -11,7 +11,7 @@
 // stores its rows itself where their bits say so: no reduction across the warp
 // per row and no replay of a batch per row, which is what k_spmm_seq spends
 // most of its instructions on when rows are short (26 warp instructions per
-// nonzero on the power-law matrix at N = 64; 10 here).  Sub-groups meet once
+// nonzero on the power-law matrix at N = 64; 11 here).  Sub-groups meet once
 // per chunk, in a segmented scan of their open partials; a range's first row,
 // begun before the range, waits for that in shared memory.  Sums are
 // deterministic: batches of U, rows in order, sub-groups in order, units in
@@ -19,10 +19,10 @@
 //
 // What bounds it: the B rows in flight per SM.  Measured, cold-to-warm L2
 // back to back, k_spmm_seq -> this form at their best unit sizes:
-//   power law 262144^2, 3.1 M nonzeros, float32: N = 64 133 -> 81 us (the
+//   power law 262144^2, 3.1 M nonzeros, float32: N = 64 133 -> 82 us (the
 //   gathers alone take 68 us), N = 32 104 -> 55, N = 8 87 -> 41, N = 128
-//   264 -> 164, N = 64 with float64 sums 210 -> 133 us;
-//   64 uneven matrices, 33 M nonzeros, N = 32: 540 -> 321 us;
+//   264 -> 164, N = 64 with float64 sums 210 -> 134 us;
+//   64 uneven matrices, 33 M nonzeros, N = 32: 540 -> 326 us;
 //   50021 x 25013, 1.2 M nonzeros, N = 33, float64 sums: 119 -> 51 us.
 #pragma once
 #include "fsb_spmm_seq.cuh"
