@@ -109,10 +109,52 @@ __device__ __forceinline__ A row_partial(const V* __restrict__ val, const I* __r
     return acc;
 }
 
+// The same for a whole warp per row (32 lanes), which rows of hundreds of
+// nonzeros take: scalar head, aligned body, scalar tail. With 128 nonzeros per
+// step the masked chunks above cost more than the two extra loops, and fewer
+// registers leave more warps to hide the loads (400000 banded rows, one in a
+// hundred of 8192 nonzeros: float32 263 us here, 273 with the chunks, float64
+// 355 and 451, bfloat16 232 and 304).
+template <class V, class A, class I>
+__device__ __forceinline__ A row_partial_wide(const V* __restrict__ val, const I* __restrict__ col,
+                                         const V* __restrict__ x, int64_t s, int64_t e,
+                                         int lane, int T, bool vec_ok) {
+    constexpr int VV = VecWidth<V>::value;
+    constexpr int VI = VecWidth<I>::value;
+    constexpr int VEC = VV < VI ? VV : VI;
+    A acc = Acc<V, A>::zero();
+    if (VEC > 1 && vec_ok) {
+        int64_t a0 = (s + VEC - 1) & ~(int64_t)(VEC - 1);
+        if (a0 > e) a0 = e;
+        int64_t a1 = e & ~(int64_t)(VEC - 1);
+        if (a1 < a0) a1 = a0;
+        for (int64_t k = s + lane; k < a0; k += T)
+            acc = Acc<V, A>::fma(ld_stream1(val + k), ld_ro1(x + idx(ld_stream1(col + k))), acc);
+#pragma unroll 2
+        for (int64_t kb = a0 + (int64_t)lane * VEC; kb < a1; kb += (int64_t)T * VEC) {
+            vec_t<V, VEC> vv = ld_stream<V, VEC>(val + kb);
+            vec_t<I, VEC> cc = ld_stream<I, VEC>(col + kb);
+            V xv[VEC];
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) xv[j] = ld_ro1(x + idx(cc.v[j]));
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) acc = Acc<V, A>::fma(vv.v[j], xv[j], acc);
+        }
+        for (int64_t k = a1 + lane; k < e; k += T)
+            acc = Acc<V, A>::fma(ld_stream1(val + k), ld_ro1(x + idx(ld_stream1(col + k))), acc);
+    } else {
+#pragma unroll 4
+        for (int64_t k = s + lane; k < e; k += T)
+            acc = Acc<V, A>::fma(ld_stream1(val + k), ld_ro1(x + idx(ld_stream1(col + k))), acc);
+    }
+    return acc;
+}
+
 template <class A> struct is_comp { static constexpr bool value = false; };
 template <> struct is_comp<comp_t> { static constexpr bool value = true; };
 
-template <class V, class A, class O, class I, class P>
+// WIDE: 32 lanes per row (lanes_log2 = 5).
+template <class V, class A, class O, class I, class P, bool WIDE>
 __global__ void __launch_bounds__(kRowsThreads)
 k_spmv_rows(const V* __restrict__ val, const I* __restrict__ col, const P* __restrict__ ptr,
             const I* __restrict__ row_map, const V* __restrict__ x, O* __restrict__ y,
@@ -132,15 +174,20 @@ k_spmv_rows(const V* __restrict__ val, const I* __restrict__ col, const P* __res
         const int64_t s = idx(ptr[row]);
         int64_t e = idx(ptr[row + 1]);
         if (row_cap > 0 && e - s > row_cap) e = s + row_cap;
+        auto partial = [&](auto ta) {
+            using B = typename decltype(ta)::type;
+            if constexpr (WIDE) return row_partial_wide<V, B, I>(val, col, x, s, e, lane, T, vec_ok);
+            else return row_partial<V, B, I>(val, col, x, s, e, nnz, lane, T, vec_ok);
+        };
         A acc;
         if constexpr (is_comp<A>::value) {
             if (e - s > comp_threshold) {
-                acc = row_partial<V, comp_t, I>(val, col, x, s, e, nnz, lane, T, vec_ok);
+                acc = partial(tag<comp_t>{});
             } else {
-                acc = comp_t{row_partial<V, float, I>(val, col, x, s, e, nnz, lane, T, vec_ok), 0.f};
+                acc = comp_t{partial(tag<float>{}), 0.f};
             }
         } else {
-            acc = row_partial<V, A, I>(val, col, x, s, e, nnz, lane, T, vec_ok);
+            acc = partial(tag<A>{});
         }
         acc = segment_reduce(mask, acc, 1, T);
         if (lane == 0) {
@@ -426,8 +473,9 @@ extern "C" int fsb_spmv_csr(const fsb_csr* A, const void* x, void* y, int out_dt
                     if (grid > 0x7fffffffLL) grid = 0x7fffffffLL;
                     const int64_t thr = plan->comp_threshold > 0 ? plan->comp_threshold : 0;
                     const int overlap = (plan->flags & FSB_PLAN_OVERLAP_LAUNCH) && grid <= kOverlapMaxBlocks;
+                    auto kern = lg == 5 ? k_spmv_rows<V, Ac, O, I, P, true> : k_spmv_rows<V, Ac, O, I, P, false>;
                     if (!overlap) {
-                        k_spmv_rows<V, Ac, O, I, P><<<(unsigned)grid, kRowsThreads, 0, st>>>(
+                        kern<<<(unsigned)grid, kRowsThreads, 0, st>>>(
                             val, col, ptr, rmap, xv, yv, A->n_rows, A->nnz, plan->row_cap, thr, lg, vec_ok, 0);
                         return fsb_host::check_launch("k_spmv_rows");
                     }
@@ -441,7 +489,7 @@ extern "C" int fsb_spmv_csr(const fsb_csr* A, const void* x, void* y, int out_dt
                     cfg.attrs = attr;
                     cfg.numAttrs = 1;
                     const int64_t nr = A->n_rows, nz = A->nnz, rc_cap = plan->row_cap;
-                    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_spmv_rows<V, Ac, O, I, P>, val, col, ptr, rmap,
+                    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, val, col, ptr, rmap,
                                                              xv, yv, nr, nz, rc_cap, thr, lg, vec_ok, 1);
                     if (e != cudaSuccess) {
                         fsb_host::set_error("k_spmv_rows (overlapped launch): %s", cudaGetErrorString(e));
