@@ -115,12 +115,17 @@ def _prepare_spmm_coo_inputs(data, row, col, B, shape):
     nnz = data.numel()
     if nnz > _INDEX_LIMIT_INT32:
         raise ValueError("nnz exceeds the int32 range supported by the Triton COO kernel")
-    # the index checks read the device: skipped while a CUDA graph records
-    # the call (the caller checks the indices before capturing)
-    data = data.contiguous()
+    # the kernels read raw memory: lazy conjugate and negative views are
+    # materialised here (contiguous() hands a contiguous lazy view back as it
+    # is); a complex32 one is refused, as its reinterpretation always was
+    if nnz > 0 and _is_complex32_dtype(data.dtype) and data.is_conj():
+        raise RuntimeError("complex32 values must not be a lazily conjugated view: pass data.resolve_conj()")
+    data = data.resolve_conj().resolve_neg().contiguous()
     row = row.contiguous()
     col = col.contiguous()
     kernel_row = kernel_col = None
+    # the index checks read the device: skipped while a CUDA graph records
+    # the call (the caller checks the indices before capturing)
     if nnz > 0 and not torch.cuda.is_current_stream_capturing():
         # the four bounds and the int32 indices in one read of both arrays
         (min_row, max_row, min_col, max_col), kernel_row, kernel_col = _nat.coo_check(row, col)
@@ -132,7 +137,7 @@ def _prepare_spmm_coo_inputs(data, row, col, B, shape):
             raise ValueError("row indices exceed the int32 range supported by the Triton kernel")
         if max_col > _INDEX_LIMIT_INT32:
             raise ValueError("column indices exceed the int32 range supported by the Triton kernel")
-    B = B.contiguous()
+    B = B.resolve_conj().resolve_neg().contiguous()
     if kernel_row is None:
         kernel_row = row.to(torch.int32) if row.dtype == torch.int64 else row
         kernel_col = col.to(torch.int32) if col.dtype == torch.int64 else col
