@@ -402,7 +402,7 @@ int launch_spmm_flat(const fsb_csr* Am, const V* val, const I* col, const P* ptr
 #undef FSB_FLAT
     int rc = fsb_host::check_launch("k_spmm_flat");
     if (rc) return rc;
-    k_spmm_merge_fixup<A, O, I, P><<<(unsigned)blocks, kSpmmThreads, 0, st>>>(
+    k_spmm_merge_fixup<A, O, I, P><<<fixup_grid(n_units, n_dense), kSpmmThreads, 0, st>>>(
         ms.carry_row, static_cast<const A*>(ms.carry_val), static_cast<const A*>(ms.head_val), n_units, n_dense, ptr,
         rmap, C, ldc);
     return fsb_host::check_launch("k_spmm_merge_fixup");
@@ -471,7 +471,7 @@ int launch_spmm(const fsb_csr* Am, const V* val, const I* col, const P* ptr, con
         ms.carry_row, static_cast<A*>(ms.carry_val), static_cast<A*>(ms.head_val));
     int rc = fsb_host::check_launch("k_spmm_merge");
     if (rc) return rc;
-    k_spmm_merge_fixup<A, O, I, P><<<(unsigned)blocks, kSpmmThreads, 0, st>>>(
+    k_spmm_merge_fixup<A, O, I, P><<<fixup_grid(n_units, n_dense), kSpmmThreads, 0, st>>>(
         ms.carry_row, static_cast<const A*>(ms.carry_val), static_cast<const A*>(ms.head_val), n_units, n_dense, ptr,
         rmap, C, ldc);
     return fsb_host::check_launch("k_spmm_merge_fixup");

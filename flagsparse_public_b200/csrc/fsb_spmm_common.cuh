@@ -41,41 +41,63 @@ __device__ __forceinline__ void zero_acc(A (&acc)[VW]) {
     for (int w = 0; w < VW; ++w) acc[w] = A{};
 }
 
-// One warp per unit: the first unit of each run carrying the same open row
-// folds the run's carries (unit order) and the ending unit's head partial.
+// The first unit of each run carrying the same open row folds the run's carries
+// (unit order) and the ending unit's head partial: one warp for all columns,
+// or, where the run goes on for kFixupLong units, one warp per 64 columns
+// (blockIdx.y).  A long run is one chain of additions per column, bound by the
+// latency of its loads: its end is looked for 128 units at a time and 64 bytes
+// of carries per lane are loaded ahead; 48 registers, since matrices of short
+// runs need the resident warps.  One row over 780 units at 1 / 33 / 128 columns,
+// a warp per run with four loads ahead -> this form, us: float32 26 / 36 / 90 ->
+// 17 / 23 / 29, float64 35 / 51 / 141 -> 29 / 39 / 60, complex128 44 / 78 / 191 ->
+// 44 / 68 / 91.  9600 rows over two units each: as before (float32 and float64
+// 6.3 at 33 columns, 8.3 at 128); a warp per 32 columns takes 7 - 8 and 10.4
+// there, 64 registers 6.6 and 8.8.
+constexpr int kFixupLong = 16;
+
 template <class A, class O, class I, class P>
-__global__ void __launch_bounds__(kSpmmThreads)
+__global__ void __launch_bounds__(kSpmmThreads, 10)
 k_spmm_merge_fixup(const int64_t* __restrict__ carry_row, const A* __restrict__ carry_val,
                    const A* __restrict__ head_val, int64_t n_units, int64_t n_dense, const P* __restrict__ ptr,
                    const I* __restrict__ row_map, O* __restrict__ C, int64_t ldc) {
+    constexpr int kAhead = 64 / (int)sizeof(A);
     const int64_t t = (int64_t)blockIdx.x * (kSpmmThreads / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (t >= n_units) return;
     const int64_t r = carry_row[t];
     if (r < 0) return;
     if (t > 0 && carry_row[t - 1] == r) return;
-    // end of the run of units carrying row r: 32 entries per step, first
-    // mismatch by ballot (a long row spans many units)
+    const bool is_long = t + kFixupLong < n_units && carry_row[t + kFixupLong] == r;
+    if (blockIdx.y > 0 && !is_long) return;
+    // end of the run of units carrying row r, by ballot (the run is one piece:
+    // full ballots, then its end, then none)
     int64_t u_end = t + 1;
-    while (true) {
-        const int64_t u = u_end + lane;
-        const bool same = u < n_units && carry_row[u] == r;
-        const unsigned stop = __ballot_sync(0xffffffffu, !same);
-        if (stop) {
-            u_end += __ffs(stop) - 1;
-            break;
+    unsigned in = 0xffffffffu;
+    while (in == 0xffffffffu) {
+        bool same[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int64_t u = u_end + i * 32 + lane;
+            same[i] = u < n_units && carry_row[u] == r;
         }
-        u_end += 32;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            in = __ballot_sync(0xffffffffu, same[i]);
+            u_end += __popc(in);
+        }
     }
     const int64_t out_row = row_map ? idx(row_map[idx(ptr[r])]) : r;
-    for (int64_t c = lane; c < n_dense; c += 32) {
-        // loads four carries ahead, adds in unit order (deterministic)
+    const int64_t step = is_long ? (int64_t)gridDim.y * 32 : 32;
+    for (int64_t c = (int64_t)blockIdx.y * 32 + lane; c < n_dense; c += step) {
+        // loads ahead, adds in unit order (deterministic)
         A sum = carry_val[t * n_dense + c];
         int64_t u = t + 1;
-        for (; u + 4 <= u_end; u += 4) {
-            const A a0 = carry_val[u * n_dense + c], a1 = carry_val[(u + 1) * n_dense + c];
-            const A a2 = carry_val[(u + 2) * n_dense + c], a3 = carry_val[(u + 3) * n_dense + c];
-            sum = acc_add(acc_add(acc_add(acc_add(sum, a0), a1), a2), a3);
+        for (; u + kAhead <= u_end; u += kAhead) {
+            A a[kAhead];
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) a[i] = carry_val[(u + i) * n_dense + c];
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) sum = acc_add(sum, a[i]);
         }
         for (; u < u_end; ++u) sum = acc_add(sum, carry_val[u * n_dense + c]);
         if (u_end < n_units) sum = acc_add(sum, head_val[u_end * n_dense + c]);
@@ -83,6 +105,11 @@ k_spmm_merge_fixup(const int64_t* __restrict__ carry_row, const A* __restrict__ 
     }
 }
 
+// Grid of k_spmm_merge_fixup.
+inline dim3 fixup_grid(int64_t n_units, int64_t n_dense) {
+    const int64_t groups = ceil_div(n_dense, (int64_t)64);
+    return dim3((unsigned)ceil_div(n_units, (int64_t)(kSpmmThreads / 32)), (unsigned)(groups < 65535 ? groups : 65535));
+}
 
 // FSB_ALGO_GATHER launch (fsb_spmm_gather.cu), dtype dispatch included.
 int spmm_gather_dispatch(const fsb_csr* A, const void* B, int64_t ldb, int64_t n_dense, void* C, int64_t ldc,

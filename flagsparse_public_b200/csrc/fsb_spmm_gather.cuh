@@ -391,7 +391,7 @@ int launch_gather(const fsb_csr* Am, const V* val, const I* col, const P* ptr, c
                                         static_cast<A*>(ms.head_val), err_word);
     int rc = fsb_host::check_launch("k_spmm_gather");
     if (rc) return rc;
-    k_spmm_merge_fixup<A, O, I, P><<<(unsigned)blocks, kSpmmThreads, 0, st>>>(
+    k_spmm_merge_fixup<A, O, I, P><<<fixup_grid(n_units, n_dense), kSpmmThreads, 0, st>>>(
         ms.carry_row, static_cast<const A*>(ms.carry_val), static_cast<const A*>(ms.head_val), n_units, n_dense, ptr,
         rmap, C, ldc);
     return fsb_host::check_launch("k_spmm_merge_fixup");

@@ -465,7 +465,7 @@ int launch_seq(const fsb_csr* Am, const V* val, const I* col, const P* ptr, cons
     }
     int rc = fsb_host::check_launch("k_spmm_seq");
     if (rc || in_kernel) return rc;
-    k_spmm_merge_fixup<A, O, I, P><<<(unsigned)blocks, kSpmmThreads, 0, st>>>(
+    k_spmm_merge_fixup<A, O, I, P><<<fixup_grid(n_units, n_dense), kSpmmThreads, 0, st>>>(
         ms.carry_row, static_cast<const A*>(ms.carry_val), static_cast<const A*>(ms.head_val), n_units, n_dense, ptr,
         rmap, C, ldc);
     return fsb_host::check_launch("k_spmm_merge_fixup");

@@ -544,11 +544,11 @@ int launch_walk(const fsb_csr* Am, const V* val, const I* col, const V* B, int64
     int rc = fsb_host::check_launch("k_spmm_walk");
     if (rc || in_kernel) return rc;
     if (ptr64)
-        k_spmm_merge_fixup<A, O, I, int64_t><<<(unsigned)blocks, kSpmmThreads, 0, st>>>(
+        k_spmm_merge_fixup<A, O, I, int64_t><<<fixup_grid(n_units, n_dense), kSpmmThreads, 0, st>>>(
             ms.carry_row, static_cast<const A*>(ms.carry_val), static_cast<const A*>(ms.head_val), n_units, n_dense,
             static_cast<const int64_t*>(Am->row_ptr), (const I*)nullptr, C, ldc);
     else
-        k_spmm_merge_fixup<A, O, I, int32_t><<<(unsigned)blocks, kSpmmThreads, 0, st>>>(
+        k_spmm_merge_fixup<A, O, I, int32_t><<<fixup_grid(n_units, n_dense), kSpmmThreads, 0, st>>>(
             ms.carry_row, static_cast<const A*>(ms.carry_val), static_cast<const A*>(ms.head_val), n_units, n_dense,
             static_cast<const int32_t*>(Am->row_ptr), (const I*)nullptr, C, ldc);
     return fsb_host::check_launch("k_spmm_merge_fixup");

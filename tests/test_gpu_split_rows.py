@@ -97,3 +97,18 @@ def test_dense_row_in_default_spmv_units(dtype):
     us = [_graph_us(lambda: _plan.run_spmv(data, col, ptr, n, n, x, y, nat.ACC_NATIVE, plan))
           for plan in (default, _plan.KernelPlan(nat.ALGO_MERGE, items_per_unit=1024))]
     assert us[0] <= 2.0 * us[1], us
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_dense_row_by_the_spmm_fixup(dtype):
+    """128 columns: the separate fix-up (one-shot products) takes no longer
+    than twice the time of the finish inside the kernel."""
+    n, n_dense = 100000, 128
+    data, col, ptr = _arrow(n, dtype)
+    B, C = torch.rand(n, n_dense, device=DEV).to(dtype), torch.empty(n, n_dense, dtype=dtype, device=DEV)
+    us = []
+    for runs in (False, None):
+        plan = _plan.default_spmm_plan(_plan.matrix_stats(ptr, n, n), n_dense, dtype)
+        plan.runs = runs
+        us.append(_graph_us(lambda: _plan.run_spmm(data, col, ptr, n, n, B, C, nat.ACC_NATIVE, plan)))
+    assert us[0] <= 2.0 * us[1], us
