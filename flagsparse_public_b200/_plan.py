@@ -293,13 +293,22 @@ def _vec_elems(dtype):
 SM_COUNT = 148  # B200
 
 
-def spmv_row_lanes(n_rows, mean, vec, skewed):
-    """Lanes per row of the row-group SpMV (the rule and its measurements:
-    spmv_row_lanes in csrc/fsb_spmv.cu, which one-shot calls use)."""
+def spmv_row_lanes(n_rows, mean, chunk, skewed):
+    """Lanes per row of the row-group SpMV; ``chunk`` elements per 16-byte step
+    of a lane (the rule and its measurements: spmv_row_lanes in
+    csrc/fsb_spmv.cu, which one-shot calls use)."""
     if skewed:
-        return _pow2_clamp(2 * mean / vec, 2, 32)
-    lanes = 2 if mean < 12.0 else 4
-    while lanes < 32 and n_rows * lanes * 2 <= SM_COUNT * 1024 and 2.0 * lanes * vec <= 2.0 * mean:
+        return 32
+    if chunk >= 4:
+        lanes = 32 if mean >= 512.0 else 16 if mean >= 200.0 else 8 if mean >= 80.0 else 4
+    elif chunk == 2:
+        lanes = 32 if mean >= 128.0 else 8 if mean >= 80.0 else 4
+    else:
+        lanes = 32 if mean >= 128.0 else 16 if mean >= 64.0 else 8 if mean >= 24.0 else 4
+    filled = n_rows * 2 >= SM_COUNT * 2048  # with two lanes per row
+    if mean < 12.0 or (filled and mean < 6.0 * chunk):
+        lanes = 2
+    while lanes < 32 and n_rows * lanes * 2 <= SM_COUNT * 1024 and 2.0 * lanes * chunk <= 2.0 * mean:
         lanes *= 2
     return lanes
 
@@ -310,18 +319,24 @@ def spmv_merge_items(n_rows, nnz):
     return _pow2_clamp((n_rows + nnz) / (SM_COUNT * 16), SPMV_MERGE_THREADS, 1024)
 
 
-def default_spmv_plan(stats, dtype, row_cap=0):
+def rows_skewed(max_row, mean):
+    """Whether a few rows dominate: the longest above 8 times the mean + 256."""
+    return max_row > 8 * max(mean, 1.0) + 256
+
+
+def default_spmv_plan(stats, dtype, row_cap=0, index_bytes=4):
     """Heuristic SpMV plan: merge path for skewed rows of less than 128
-    nonzeros on average (longer average rows keep 16-32 lanes busy even when a
-    few rows are much longer), else row groups of few lanes.  The same choice
-    as checked_plan in csrc/fsb_spmv.cu."""
+    nonzeros on average, else row groups.  The same choice as checked_plan in
+    csrc/fsb_spmv.cu."""
     if row_cap > 0 or stats.n_rows == 0:
         lanes = _pow2_clamp(stats.mean_row / _vec_elems(dtype), 2, 32) if stats.n_rows else 32
         return KernelPlan(nat.ALGO_ROWS, lanes=lanes, row_cap=row_cap)
-    skewed = stats.max_row > 8 * max(stats.mean_row, 1.0) + 256
-    if skewed and stats.mean_row < 128.0:
+    mean = stats.mean_row
+    chunk = 16 // max(dtype.itemsize, index_bytes)
+    skewed = rows_skewed(stats.max_row, mean)
+    if skewed and mean < 128.0:
         return KernelPlan(nat.ALGO_MERGE, items_per_unit=spmv_merge_items(stats.n_rows, stats.nnz))
-    lanes = spmv_row_lanes(stats.n_rows, stats.mean_row, _vec_elems(dtype), skewed)
+    lanes = spmv_row_lanes(stats.n_rows, mean, chunk, skewed)
     return KernelPlan(nat.ALGO_ROWS, lanes=lanes, flags=nat.PLAN_OVERLAP_LAUNCH)
 
 

@@ -15,6 +15,7 @@
 // FlagSparse computes the same products in _spmv_csr_real_kernel
 // (spmv_csr.py:158-184), _spmv_csr_complex_kernel (:187-219), the CSR-vector
 // bucket kernels (:225-343) and the COO row-run kernels (spmv_coo.py:131-226).
+#include <algorithm>
 #include <cstring>
 #include <cmath>
 #include <mutex>
@@ -592,24 +593,45 @@ extern "C" int fsb_spmv_csr(const fsb_csr* A, const void* x, void* y, int out_dt
 namespace {
 int64_t check_bytes(const fsb_csr* A) { return align_up(fsb_csr_check_workspace_bytes(A->n_rows, A->nnz), 256); }
 
-// Lanes of a row group: 2 for rows of less than 12 nonzeros on average, else
-// 4; wider while the whole grid would hold at most 1024 threads per SM and the
-// lanes' chunks stay below twice the row.  Rows that a few long ones dominate
-// (skewed, 128 nonzeros or more on average) take 2 * mean / (16-byte vector
-// elements) lanes.  Measured (us, lanes 2 / 4 / 8 / 16 / 32, float32):
-// 10^6 rows of 4 31 / 45 / 88 / 176 / 359, 10^6 of 8 44 / 58 / 97 / 190 / 390,
-// 10^5 of 23 15 / 13 / 14 / 20 / 38, 5 * 10^5 of 48 113 / 106 / 112 / 142 /
-// 226, 10^5 of 128 48 / 38 / 47 / 54 / 65, 16384 of 16 4.2 / 3.6 / 3.4 / 4.8 /
-// 7.9 (default_spmv_plan in _plan.py follows the same rule).
-int spmv_row_lanes(int64_t n_rows, double mean, int vec, bool skewed) {
-    if (skewed) {
-        double v = 2.0 * mean / vec;
-        if (v < 1.0) v = 1.0;
-        const int lanes = 1 << (int)std::nearbyint(std::log2(v));
-        return lanes < 2 ? 2 : (lanes > 32 ? 32 : lanes);
-    }
-    int lanes = mean < 12.0 ? 2 : 4;
-    while (lanes < 32 && n_rows * lanes * 2 <= 148 * 1024 && 2.0 * lanes * vec <= 2.0 * mean) lanes *= 2;
+// Lanes of a row group.  `chunk` is the elements of one 16-byte step of a lane
+// (spmv_chunk: the smaller of the value and the index vector); a lane should have a few
+// whole steps of its row, and a row of hundreds of nonzeros a whole warp:
+//   chunk 4 (32-bit indices, values up to 4 bytes): 2 lanes, 4 from 12 (24
+//           where the rows alone fill the chip) nonzeros on average, 8 from
+//           80, 16 from 200, 32 from 512;
+//   chunk 2 (8-byte values or indices): 2, 4 from 12, 8 from 80, 32 from 128;
+//   chunk 1 (16-byte values): 2, 4 from 12, 8 from 24, 16 from 64, 32 from 128;
+// doubled while the whole grid would hold at most 1024 threads per SM and the
+// lanes' steps stay below twice the row.
+// Measured, kernel us at lanes 2 / 4 / 8 / 16 / 32 (rows x mean, Poisson):
+//   float32  10^6 x 4 32 / 48 / 86 / 166 / 285, 10^6 x 16 78 / 85 / 111 / 190 / 366,
+//            10^5 x 12 8.8 / 8.7 / 10.7 / 17.6 / 36, 10^5 x 64 36 / 30 / 29 / 32 / 45,
+//            10^5 x 150 80 / 62 / 59 / 60 / 73, 10^5 x 300 154 / 113 / 109 / 102 / 109,
+//            20000 x 1000 95 / 54 / 54 / 44 / 42, 5000 x 3000 - / 94 / 56 / 34 / 33;
+//   float16  10^6 x 12 64 / 76 / 109 / 199 / 368, 20000 x 1000 107 / 60 / 59 / 47 / 37;
+//            64-bit indices: 20000 x 1000 179 / 95 / 58 / 54 / 43;
+//   float64  10^5 x 32 28 / 22 / 23 / 27 / 39, 10^5 x 100 81 / 60 / 57 / 59 / 66,
+//            50000 x 150 52 / 51 / 41 / 42 / 39, 20000 x 1000 235 / 122 / 126 / 93 / 56;
+//   complex128 10^5 x 12 12 / 11 / 12 / 16 / 27, 50000 x 32 17 / 13 / 12 / 13 / 18,
+//            10^5 x 64 60 / 48 / 41 / 40 / 48, 10^5 x 300 266 / 192 / 166 / 153 / 146.
+// Four lanes for every row from 12 on (no step up with the mean) took up to
+// 2.1 times the time of 32 on rows of 1000 (10^4 rows, 16-bit values, 64-bit
+// indices: 50 us, 25 with 32 lanes).
+// Rows that a few long ones dominate (skewed, off the merge path) take a whole
+// warp.  default_spmv_plan in _plan.py follows the same rule.
+int spmv_chunk(int value_bytes, int index_bytes) {
+    return 16 / std::max(1, std::min(16, std::max(value_bytes, index_bytes)));
+}
+
+int spmv_row_lanes(int64_t n_rows, double mean, int chunk, bool skewed) {
+    if (skewed) return 32;
+    int lanes;
+    if (chunk >= 4) lanes = mean >= 512.0 ? 32 : (mean >= 200.0 ? 16 : (mean >= 80.0 ? 8 : 4));
+    else if (chunk == 2) lanes = mean >= 128.0 ? 32 : (mean >= 80.0 ? 8 : 4);
+    else lanes = mean >= 128.0 ? 32 : (mean >= 64.0 ? 16 : (mean >= 24.0 ? 8 : 4));
+    const bool filled = n_rows * 2 >= 148 * 2048;  // with two lanes per row
+    if (mean < 12.0 || (filled && mean < 6.0 * chunk)) lanes = 2;
+    while (lanes < 32 && n_rows * lanes * 2 <= 148 * 1024 && 2.0 * lanes * chunk <= 2.0 * mean) lanes *= 2;
     return lanes;
 }
 
@@ -628,8 +650,7 @@ int32_t spmv_merge_items(const fsb_csr* A) {
 // on average (Zipf rows of 40: row groups 227 us, merge path 61).
 void checked_plan(const fsb_csr* A, const int64_t* fig, fsb_plan* plan) {
     memset(plan, 0, sizeof(*plan));
-    const int esz = elem_size(A->value_dtype);
-    const int vec = esz >= 16 ? 1 : 16 / esz;
+    const int chunk = spmv_chunk(elem_size(A->value_dtype), elem_size(A->index_dtype));
     const double mean = A->n_rows ? (double)A->nnz / (double)A->n_rows : 0.0;
     const bool skewed = (double)fig[5] > 8.0 * (mean > 1.0 ? mean : 1.0) + 256.0;
     if (A->n_rows > 0 && skewed && mean < 128.0) {
@@ -639,7 +660,7 @@ void checked_plan(const fsb_csr* A, const int64_t* fig, fsb_plan* plan) {
         return;
     }
     plan->algo = FSB_ALGO_ROWS;
-    plan->lanes = A->n_rows ? spmv_row_lanes(A->n_rows, mean, vec, skewed) : 32;
+    plan->lanes = A->n_rows ? spmv_row_lanes(A->n_rows, mean, chunk, skewed) : 32;
     plan->flags = FSB_PLAN_OVERLAP_LAUNCH;
 }
 

@@ -104,7 +104,8 @@ def _mixed_plan(prepared, kind, n_dense=0, operands=None):
     if plan is None:
         st = _stats(prepared)
         if kind == "spmv":
-            plan = _plan.default_spmv_plan(st, prepared.data.dtype)
+            plan = _plan.default_spmv_plan(st, prepared.data.dtype,
+                                           index_bytes=prepared.kernel_indices.element_size())
         elif operands is not None:
             B, C = operands
             plan = _plan.chosen_spmm_plan(st, prepared.data, prepared.kernel_indices, prepared.kernel_indptr,

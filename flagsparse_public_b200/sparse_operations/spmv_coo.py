@@ -250,7 +250,8 @@ def _coo_run_plan(prepared):
     if prepared._plan is None:
         n, nnz = prepared.n_rows, prepared.nnz
         stats = _plan.MatrixStats(n, prepared.n_cols, nnz, nnz, nnz / max(n, 1), 0.0, 0)
-        prepared._plan = _plan.default_spmv_plan(stats, prepared.data.dtype)
+        prepared._plan = _plan.default_spmv_plan(stats, prepared.data.dtype,
+                                                 index_bytes=prepared.col.element_size())
     return prepared._plan
 
 

@@ -158,7 +158,8 @@ def _spmv_plan(prepared, kind, row_cap=0):
     key = (kind, int(row_cap))
     plan = prepared._plans.get(key)
     if plan is None:
-        plan = _plan.default_spmv_plan(_spmv_stats(prepared), prepared.data.dtype, row_cap=row_cap)
+        plan = _plan.default_spmv_plan(_spmv_stats(prepared), prepared.data.dtype, row_cap=row_cap,
+                                       index_bytes=prepared.kernel_indices.element_size())
         prepared._plans[key] = plan
     return plan
 
