@@ -325,16 +325,17 @@ def rows_skewed(max_row, mean):
 
 
 def default_spmv_plan(stats, dtype, row_cap=0, index_bytes=4):
-    """Heuristic SpMV plan: merge path for skewed rows of less than 128
-    nonzeros on average, else row groups.  The same choice as checked_plan in
-    csrc/fsb_spmv.cu."""
+    """Heuristic SpMV plan: merge path for skewed rows that are short on
+    average (or of medium length in a large matrix or beside a very long row),
+    else row groups.  The same choice as checked_plan in csrc/fsb_spmv.cu,
+    where the limits are explained."""
     if row_cap > 0 or stats.n_rows == 0:
         lanes = _pow2_clamp(stats.mean_row / _vec_elems(dtype), 2, 32) if stats.n_rows else 32
         return KernelPlan(nat.ALGO_ROWS, lanes=lanes, row_cap=row_cap)
     mean = stats.mean_row
     chunk = 16 // max(dtype.itemsize, index_bytes)
     skewed = rows_skewed(stats.max_row, mean)
-    if skewed and mean < 128.0:
+    if skewed and (mean < 32.0 or (mean < 128.0 and (stats.nnz >= 1 << 21 or stats.max_row > 32 * 32 * chunk))):
         return KernelPlan(nat.ALGO_MERGE, items_per_unit=spmv_merge_items(stats.n_rows, stats.nnz))
     lanes = spmv_row_lanes(stats.n_rows, mean, chunk, skewed)
     return KernelPlan(nat.ALGO_ROWS, lanes=lanes, flags=nat.PLAN_OVERLAP_LAUNCH)

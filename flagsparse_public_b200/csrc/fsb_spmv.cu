@@ -646,14 +646,21 @@ int32_t spmv_merge_items(const fsb_csr* A) {
 }
 
 // Row groups or merge path from the check's figures: merge path for skewed
-// rows (the longest above 8 times the mean + 256) of less than 128 nonzeros
-// on average (Zipf rows of 40: row groups 227 us, merge path 61).
+// rows (the longest above 8 times the mean + 256) of less than 32 nonzeros on
+// average, or of less than 128 where the matrix has at least 2^21 nonzeros or
+// the longest row more than 32 steps of a whole warp (Zipf rows of 40, 12 M
+// nonzeros: row groups 227 us, merge path 61).  A small matrix without such a
+// row stays with the row groups there: the merge path's second launch and its
+// workspace cost more than the balance gains (a prepared call, 2000 rows of 100
+// with the longest at 2000: float32 14.7 us, 21.4 on the merge path, complex128
+// 25 and 21; with the longest at 20000 the kernels alone 57 us and 9).
 void checked_plan(const fsb_csr* A, const int64_t* fig, fsb_plan* plan) {
     memset(plan, 0, sizeof(*plan));
     const int chunk = spmv_chunk(elem_size(A->value_dtype), elem_size(A->index_dtype));
     const double mean = A->n_rows ? (double)A->nnz / (double)A->n_rows : 0.0;
     const bool skewed = (double)fig[5] > 8.0 * (mean > 1.0 ? mean : 1.0) + 256.0;
-    if (A->n_rows > 0 && skewed && mean < 128.0) {
+    if (A->n_rows > 0 && skewed &&
+        (mean < 32.0 || (mean < 128.0 && (A->nnz >= (1 << 21) || fig[5] > 32 * 32 * chunk)))) {
         plan->algo = FSB_ALGO_MERGE;
         plan->items_per_unit = spmv_merge_items(A);
         plan->n_units = ceil_div(A->n_rows + A->nnz, plan->items_per_unit);

@@ -245,8 +245,10 @@ def _coo_row_ptr(prepared):
 
 def _coo_run_plan(prepared):
     """Plan from the sizes the host knows: the longest row is taken as
-    unknown (as long as all nonzeros), so short-row matrices go merge path,
-    which is balanced whatever the row lengths."""
+    unknown (as long as all nonzeros), so matrices of less than 128 nonzeros
+    per row go merge path, which is balanced whatever the row lengths: 20000
+    even rows of 48 cost 24 us a call and not 19 as row groups, 20000 Zipf rows
+    of 48 14 us of kernel time and not 111."""
     if prepared._plan is None:
         n, nnz = prepared.n_rows, prepared.nnz
         stats = _plan.MatrixStats(n, prepared.n_cols, nnz, nnz, nnz / max(n, 1), 0.0, 0)
@@ -263,14 +265,15 @@ def _triton_spmv_coo_kernel(prepared, x, block_size, num_warps, block_inner):
     """
     del block_size, num_warps, block_inner
     dtype = prepared.data.dtype
-    y = torch.zeros(prepared.n_rows, dtype=dtype, device=prepared.data.device)
-    if prepared.nnz == 0:
-        return y
-    if prepared.use_seg_kernel:
+    if prepared.nnz > 0 and prepared.use_seg_kernel:
         # the row runs as rows of a CSR structure over all rows: each run's
-        # sum in entry order, empty rows 0
+        # sum in entry order, empty rows 0 (every row is written)
+        y = torch.empty(prepared.n_rows, dtype=dtype, device=prepared.data.device)
         _plan.run_spmv(prepared.data, prepared.col, _coo_row_ptr(prepared), prepared.n_rows, prepared.n_cols, x, y,
                        _nat.ACC_NATIVE, _coo_run_plan(prepared))
+        return y
+    y = torch.zeros(prepared.n_rows, dtype=dtype, device=prepared.data.device)
+    if prepared.nnz == 0:
         return y
     lib = _nat.library()
     row = prepared.row if prepared.row.dtype == prepared.col.dtype else prepared.row.to(prepared.col.dtype)

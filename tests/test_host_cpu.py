@@ -190,6 +190,23 @@ def test_default_plans():
     assert capped.algo == nat.ALGO_ROWS and capped.row_cap == 32
 
 
+def test_spmv_merge_path_needs_a_long_row_or_a_large_matrix():
+    """Skewed rows of 32 to 128 nonzeros: a small matrix without a very long
+    row keeps the row groups (a whole warp each)."""
+    def plan(rows, mean, max_row, dtype=torch.float32, index_bytes=4):
+        stats = _plan.MatrixStats(rows, rows, rows * mean, max_row, float(mean), 0.0, 0)
+        return _plan.default_spmv_plan(stats, dtype, index_bytes=index_bytes)
+
+    small = plan(2000, 100, 2000)
+    assert small.algo == nat.ALGO_ROWS and small.lanes == 32
+    assert plan(2000, 100, 4097).algo == nat.ALGO_MERGE  # more than 32 steps of 128
+    assert plan(2000, 100, 2000, torch.complex128).algo == nat.ALGO_MERGE  # 62 steps of 32
+    assert plan(2000, 100, 2000, index_bytes=8).algo == nat.ALGO_ROWS  # 31 steps of 64
+    assert plan(30000, 100, 2000).algo == nat.ALGO_MERGE  # 3 M nonzeros
+    assert plan(2000, 30, 2000).algo == nat.ALGO_MERGE  # short rows
+    assert plan(30000, 128, 20000).algo == nat.ALGO_ROWS  # long rows
+
+
 def test_batch_stacking_is_block_diagonal():
     from flagsparse_public_b200 import batched, synthetic
     mats = [synthetic.poisson_uniform(r, c, mean=m, seed=s, device="cpu")
