@@ -302,7 +302,7 @@ k_spmv_merge(const V* __restrict__ val, const I* __restrict__ col, const P* __re
             const bool in = row < n_rel;
             const int s = in ? start_of(row) : 0, e = in ? start_of(row + 1) : 0;
             const bool take = in && (s < end || (last && row < n_ends));
-            if (take && e > s && s >= 0 && s < end) {
+            if (take && e > s && s >= (kc < 0 ? 0 : kc) && s < end) {
                 s_row[s - kc] = row + 1;
                 s_flag[s - kc] = 1;
             }
