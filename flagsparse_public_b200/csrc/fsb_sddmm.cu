@@ -3,8 +3,8 @@
 // for every stored position p (FlagSparse's flagsparse_sddmm_csr,
 // sddmm_csr.py:350-422, kernel _sddmm_csr_real_kernel :108-152).
 //
-// A sub-group of LPN lanes computes kSddmmU consecutive positions at a time,
-// each lane covering VW consecutive elements of K per step (16-byte vectors
+// A sub-group of LPN lanes computes kSddmmU positions at a time (consecutive
+// ones, in sub-groups of one or two lanes ones a warp's width apart), each lane covering VW consecutive elements of K per step (16-byte vectors
 // where x and y allow).  The positions' indices come as vector loads, their y
 // rows are loaded back to back (random gathers, latency bound), and x is
 // loaded once where the positions of every sub-group lie in one row each.  The
@@ -41,10 +41,20 @@ __device__ __forceinline__ void load_indices(const I* __restrict__ a, int64_t p0
 
 // What bounds it: y rows in flight per SM.  Power-law pattern, 3.1 M
 // positions, before (a reduction per position, x loaded per position) -> now:
-// float32 K = 64 144 -> 130 us (its gathers alone: 68), K = 128 299 -> 251, K =
-// 143 (single elements) 598 -> 482, K = 200 754 -> 497; float64 K = 64 434 ->
-// 281.  Eight positions per batch: 151 us at 2 CTAs (128 registers), 186 at 3
-// (spills); 3 or 5 CTAs with four: 166 and 136.
+// float32 K = 64 144 -> 119 us (its gathers alone: 68); 3.2 M positions,
+// float32 K = 33 (single elements) 357 -> 265, K = 128 303 -> 255, K = 200 749 -> 503;
+// float64 K = 64 435 -> 283, K = 200 1185 -> 811.  Eight positions per batch: 151 us
+// at 2 CTAs (128 registers), 186 at 3 (spills); 3 or 5 CTAs with four: 166 and
+// 136 (all three with the loop over K that one step has since replaced below
+// 32 lanes).
+// Sub-groups of one or two lanes (K up to two vectors) take positions NPAR
+// apart: with neighbouring ones per lane every index load and store of the
+// warp spreads over four times the lines (3 M positions, kernel us, a
+// reduction per position / neighbouring / apart: float64 K = 1 15.6 / 24 /
+// 15.7, float32 K = 4 16.6 / 18 / 16.1, K = 2 16.4 / 17.1 / 14.5).
+// Below 32 lanes the lanes cover K in one step: without the loop the compiler
+// spends no registers on unrolling it (float32 K = 64 114 -> 101 us on even
+// rows, K = 2 21.6 -> 14.5).
 template <class V, class A, class I, int VW, int LPN_LOG2>
 __global__ void __launch_bounds__(kSddmmThreads, 4)
 k_sddmm(const I* __restrict__ col, const int32_t* __restrict__ row_ids, int64_t nnz, const V* __restrict__ x,
@@ -55,25 +65,37 @@ k_sddmm(const I* __restrict__ col, const int32_t* __restrict__ row_ids, int64_t 
     constexpr int U = kSddmmU;
     constexpr int HALVINGS = LPN_LOG2 < 2 ? LPN_LOG2 : 2;  // log2 U at most
     constexpr int LEFT = U >> HALVINGS;  // results per storing lane
+    constexpr bool kApart = LPN_LOG2 <= 1;
     constexpr unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int sub = lane >> LPN_LOG2, cl = lane & (LPN - 1);
     const int64_t warp = ((int64_t)blockIdx.x * kSddmmThreads + threadIdx.x) >> 5;
     const int64_t n_warps = ((int64_t)gridDim.x * kSddmmThreads) >> 5;
     for (int64_t base = warp * (NPAR * U); base < nnz; base += n_warps * (NPAR * U)) {
-        const int64_t p0 = base + sub * U;
+        // the sub-group's positions: U consecutive ones, or (kApart) NPAR apart
+        const int64_t p0 = base + (kApart ? sub : sub * U);
         I c[U];
         int32_t r[U];
-        load_indices<I>(col, p0, nnz, vec_ok, c);
-        load_indices<int32_t>(row_ids, p0, nnz, vec_ok, r);
-        bool same = true;
+        bool one_row = false;
+        if constexpr (kApart) {
 #pragma unroll
-        for (int u = 1; u < U; ++u) same = same && r[u] == r[0];
-        const bool one_row = __all_sync(full, same);
+            for (int u = 0; u < U; ++u) {
+                const int64_t p = p0 + u * NPAR < nnz ? p0 + u * NPAR : nnz - 1;
+                c[u] = col[p];
+                r[u] = row_ids[p];
+            }
+        } else {
+            load_indices<I>(col, p0, nnz, vec_ok, c);
+            load_indices<int32_t>(row_ids, p0, nnz, vec_ok, r);
+            bool same = true;
+#pragma unroll
+            for (int u = 1; u < U; ++u) same = same && r[u] == r[0];
+            one_row = __all_sync(full, same);
+        }
         A acc[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) acc[u] = A(0);
-        for (int64_t kk = (int64_t)cl * VW; kk < k; kk += (int64_t)LPN * VW) {
+        auto step = [&](int64_t kk) {
             vec_t<V, VW> yv[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) yv[u] = ld_ro<V, VW>(y + idx(c[u]) * ldy + kk);
@@ -92,6 +114,11 @@ k_sddmm(const I* __restrict__ col, const int32_t* __restrict__ row_ids, int64_t 
 #pragma unroll
                     for (int w = 0; w < VW; ++w) acc[u] = fma((A)xv[u].v[w], (A)yv[u].v[w], acc[u]);
             }
+        };
+        if constexpr (LPN_LOG2 < 5) {  // the lanes cover k in one step
+            if (cl * VW < k) step(cl * VW);
+        } else {
+            for (int64_t kk = (int64_t)cl * VW; kk < k; kk += (int64_t)LPN * VW) step(kk);
         }
         // halving steps: the upper half of the lanes keeps the upper half of
         // the sums, the lower half the lower
@@ -113,7 +140,7 @@ k_sddmm(const I* __restrict__ col, const int32_t* __restrict__ row_ids, int64_t 
         if ((cl & ((LPN >> HALVINGS) - 1)) == 0) {
 #pragma unroll
             for (int i = 0; i < LEFT; ++i) {
-                const int64_t p = p0 + first + i;
+                const int64_t p = p0 + (first + i) * (kApart ? NPAR : 1);
                 if (p < nnz) {
                     A v = alpha * acc[i];
                     if (data) v += (A)data[p] * beta;

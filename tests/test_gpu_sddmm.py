@@ -72,3 +72,29 @@ def test_validation_messages_match_flagsparse():
         flagsparse_sddmm_csr(None, ind, ptr, x, y[:, :3], (2, 3))
     out = flagsparse_sddmm_csr(None, ind, ptr, x[:, :0], y[:, :0], (2, 3))
     assert torch.all(out == 0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 8, 16, 33, 64])
+def test_positions_at_the_ends_of_a_batch(dtype, k):
+    """Position counts around a sub-group's four and a warp's batch, with the
+    pattern's indices on and off the 16-byte grid (their vector and single
+    loads): sub-groups of one and two lanes take positions apart, wider ones
+    neighbouring ones."""
+    g = torch.Generator().manual_seed(k)
+    n_rows, n_cols = 40, 23
+    x = torch.randn((n_rows, k), generator=g, dtype=torch.float64).to(dtype)
+    y = torch.randn((n_cols, k), generator=g, dtype=torch.float64).to(dtype)
+    for nnz in (1, 3, 4, 5, 15, 16, 17, 63, 64, 65, 127, 128, 129, 515):
+        rows = torch.sort(torch.randint(0, n_rows, (nnz,), generator=g)).values
+        indptr = torch.zeros(n_rows + 1, dtype=torch.int64)
+        indptr[1:] = torch.cumsum(torch.bincount(rows, minlength=n_rows), 0)
+        indices = torch.randint(0, n_cols, (nnz,), generator=g, dtype=torch.int32)
+        data = torch.randn(nnz, generator=g, dtype=torch.float64).to(dtype)
+        exact, mag = exact_sddmm({"indptr": indptr, "indices": indices, "x": x, "y": y, "alpha": 1.5, "beta": -0.25,
+                                  "has_data": True, "data": data})
+        for shift in (0, 1):
+            idx = torch.cat([torch.zeros(shift, dtype=torch.int32), indices]).to(DEV)[shift:]
+            prep = prepare_sddmm_csr(idx, indptr.to(DEV), (n_rows, n_cols), k_hint=k)
+            out = flagsparse_sddmm_csr(data.to(DEV), x=x.to(DEV), y=y.to(DEV), prepared=prep, alpha=1.5, beta=-0.25)
+            assert _err(out, exact, mag) <= (3e-5 if dtype == torch.float32 else 1e-12), (nnz, shift)
