@@ -362,14 +362,51 @@ def walk_items_per_unit(n_rows, nnz):
     return _pow2_clamp((int(n_rows) + int(nnz)) / (SM_COUNT * WALK_WARPS_PER_SM), 128, 1024)
 
 
-def default_spmm_plan(stats, n_dense, dtype, row_cap=0):
+def spmm_form(n_dense, dtype, mean, skewed):
+    """PLAN_WALK where the range-walk form of the merge-path SpMM is the faster
+    one, 0 for k_spmm_seq.  At up to four columns the walk's sub-groups have
+    one or two batches of a chunk each and their meeting costs more than the
+    warp-wide reduction of a long row in k_spmm_seq.  Seq over walk time (even
+    rows of 60 / 100 / 400 nonzeros): complex128 0.58 / 0.64 / 0.53 at one
+    column, 0.70 / 0.74 / 0.62 at four; float64 0.85 / 1.02 / 0.98 at one, 0.83
+    / 0.94 / 0.82 at two, 0.81 / 0.92 / 0.78 at four; complex64 0.87 / 1.07 /
+    0.99, 0.85 / 1.09 / 0.95 and 0.85 / 1.01 / 0.87; three columns (no lane
+    vectors) float64 0.69 / 0.81 / 0.67, complex64 0.72 / 0.81 / 0.73, float32
+    0.90 / 1.00 / 0.93.  Rows of 20: complex128 0.71, float64 1.2 - 1.3; power-law
+    rows of 100: complex128 0.78, float64 1.24 / 1.14 / 0.85 / 1.12 at one to
+    four columns; rows of 5 at least 1.5 in every type."""
+    if n_dense > 4 or mean < (20.0 if dtype == torch.complex128 else 40.0):
+        return nat.PLAN_WALK
+    if dtype == torch.complex128 or (n_dense == 3 and (dtype.itemsize >= 8 or not skewed)):
+        return 0
+    return 0 if dtype == torch.float64 and n_dense > 1 and not skewed else nat.PLAN_WALK
+
+
+def fit_form(plan, row_ptr, n_rows, nnz, n_dense, dtype):
+    """``plan`` (a SEQ plan made for the range walk, or another one, returned
+    as it is) in the form that spmm_form picks; reads the longest row from the
+    device where that decides."""
+    if not (isinstance(plan, KernelPlan) and plan.flags & nat.PLAN_WALK) or n_dense > 4 or n_rows == 0:
+        return plan
+    mean = nnz / n_rows
+    forms = [spmm_form(n_dense, dtype, mean, skewed) for skewed in (False, True)]
+    form = forms[0]
+    if forms[0] != forms[1]:
+        form = forms[rows_skewed(int((row_ptr[1:] - row_ptr[:-1]).max()), mean)]
+    plan.flags = (plan.flags & ~nat.PLAN_WALK) | form
+    return plan
+
+
+def default_spmm_plan(stats, n_dense, dtype, row_cap=0, acc_mode=nat.ACC_NATIVE):
     """Heuristic SpMM plan: the batched merge-path kernel (nonzero-balanced
     units, rows split across units where long); row groups when a per-row
-    segment cap is requested."""
+    segment cap is requested.  Compensated sums run in k_spmm_seq."""
     if row_cap > 0 or stats.n_rows == 0:
         return KernelPlan(nat.ALGO_ROWS, lanes=32, row_cap=row_cap)
-    return KernelPlan(nat.ALGO_SEQ, items_per_unit=seq_items_per_unit(stats), snap=SPMM_SNAP_DEFAULT,
-                      flags=nat.PLAN_WALK)
+    form = 0
+    if acc_mode != nat.ACC_COMP:
+        form = spmm_form(n_dense, dtype, stats.mean_row, rows_skewed(stats.max_row, stats.mean_row))
+    return KernelPlan(nat.ALGO_SEQ, items_per_unit=seq_items_per_unit(stats), snap=SPMM_SNAP_DEFAULT, flags=form)
 
 
 # How the prepared SpMM paths pick their plan: "learned" (the shipped
@@ -422,12 +459,12 @@ def chosen_spmm_plan(stats, data, indices, indptr, n_rows, n_cols, B, C, acc_mod
     n_dense = int(B.shape[1])
     mode = _selector_mode
     if mode == "heuristic" or stats.n_rows == 0 or n_dense == 0:
-        return default_spmm_plan(stats, n_dense, data.dtype)
+        return default_spmm_plan(stats, n_dense, data.dtype, acc_mode=acc_mode)
     if mode == "learned":
         sel = learned_selector(B.device)
         if sel is not None:
             return sel.select(data, indices, indptr, n_rows, n_cols, B, C, acc_mode)
-        return default_spmm_plan(stats, n_dense, data.dtype)
+        return default_spmm_plan(stats, n_dense, data.dtype, acc_mode=acc_mode)
     plan, _ = _tuner().tune(data, indices, indptr, n_rows, n_cols, B, C, acc_mode)
     return plan
 

@@ -95,6 +95,7 @@ class PreparedCsrBatch:
                 plan = BATCH_CANDIDATES[best][1]()
             else:
                 plan = BATCH_CANDIDATES[0][1]()
+            plan = _plan.fit_form(plan, self.indptr, self.n_rows, self.nnz, self.n_dense, dtype)
         self.plan = plan
         self.plan.ensure_coords(self.indptr, self.n_rows, self.nnz)
         self.graph = None

@@ -111,7 +111,7 @@ def _mixed_plan(prepared, kind, n_dense=0, operands=None):
             plan = _plan.chosen_spmm_plan(st, prepared.data, prepared.kernel_indices, prepared.kernel_indptr,
                                           prepared.n_rows, prepared.n_cols, B, C, _acc_mode(prepared))
         else:
-            plan = _plan.default_spmm_plan(st, n_dense, prepared.data.dtype)
+            plan = _plan.default_spmm_plan(st, n_dense, prepared.data.dtype, acc_mode=_acc_mode(prepared))
         plan.comp_threshold = prepared.compensate_above
         prepared._plans[key] = plan
     return plan

@@ -153,7 +153,7 @@ def time_candidates(data, indices, indptr, n_rows, n_cols, B, C, acc_mode, candi
     touch), then ``reps`` timed calls (one when a call takes > slow_ms)."""
     times = []
     for _name, make in candidates:
-        plan = make()
+        plan = _plan.fit_form(make(), indptr, n_rows, data.numel(), B.shape[1], data.dtype)
         run = lambda: _plan.run_spmm(data, indices, indptr, n_rows, n_cols, B, C, acc_mode, plan)  # noqa: E731
         try:
             _time_ms(run, 1)  # untimed: one-time costs
@@ -186,7 +186,8 @@ class Autotuner:
             best = int(np.argmin(times))
             hit = (best, dict(zip(CANDIDATE_NAMES, times)))
             self.cache[k] = hit
-        return SPMM_CANDIDATES[hit[0]][1](), hit[1]
+        plan = _plan.fit_form(SPMM_CANDIDATES[hit[0]][1](), indptr, n_rows, data.numel(), B.shape[1], data.dtype)
+        return plan, hit[1]
 
 
 # --------------------------------------------------------------------- MLP

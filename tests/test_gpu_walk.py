@@ -16,6 +16,7 @@ from flagsparse_public_b200 import _plan
 from oracle import oracle as orc
 from tests.gpu_cases import csr_from_lengths, dense
 from tests.numerics import REL_BOUND, scaled_error
+from tests.test_gpu_split_rows import _graph_us
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -81,3 +82,22 @@ def test_walk_leaves_non_finite_b_rows_alone():
     _plan.run_spmm(data.to(DEV), indices.to(DEV), indptr.to(DEV), n_rows, n_cols, B.to(DEV), C, nat.ACC_NATIVE,
                    _plan.KernelPlan(nat.ALGO_SEQ, items_per_unit=128, flags=nat.PLAN_WALK))
     assert scaled_error(C, exact, mag) <= 3e-5
+
+
+@pytest.mark.parametrize("dtype,n_dense,mean", [(torch.complex128, 1, 400), (torch.complex128, 4, 60),
+                                                (torch.float64, 3, 400), (torch.float64, 4, 100),
+                                                (torch.float32, 32, 60), (torch.float64, 8, 20)])
+def test_default_form_is_the_faster_one(dtype, n_dense, mean):
+    """The default plan's form takes at most 1.15 times the other one."""
+    rows = 20000
+    ptr = torch.arange(rows + 1, device=DEV) * mean
+    col = torch.randint(0, rows, (rows * mean,), device=DEV, dtype=torch.int32)
+    data, B = torch.ones(rows * mean, dtype=dtype, device=DEV), torch.ones(rows, n_dense, dtype=dtype, device=DEV)
+    C = torch.empty_like(B)
+    st = _plan.matrix_stats(ptr, rows, rows)
+    default = _plan.default_spmm_plan(st, n_dense, dtype)
+    other = _plan.KernelPlan(nat.ALGO_SEQ, snap=default.snap, flags=default.flags ^ nat.PLAN_WALK,
+                             items_per_unit=default.items_per_unit)
+    us = [_graph_us(lambda: _plan.run_spmm(data, col, ptr, rows, rows, B, C, nat.ACC_NATIVE, plan))
+          for plan in (default, other)]
+    assert us[0] <= 1.15 * us[1], us

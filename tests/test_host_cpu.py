@@ -207,6 +207,25 @@ def test_spmv_merge_path_needs_a_long_row_or_a_large_matrix():
     assert plan(30000, 128, 20000).algo == nat.ALGO_ROWS  # long rows
 
 
+def test_spmm_form_of_narrow_operands():
+    """Up to four columns with long rows run in k_spmm_seq where that is the
+    faster form, as compensated sums do; all else in the range walk."""
+    walk, form = nat.PLAN_WALK, _plan.spmm_form
+    for n in (5, 8, 64):
+        assert form(n, torch.complex128, 400.0, False) == walk
+    for n in (1, 2, 3, 4):
+        assert form(n, torch.complex128, 20.0, True) == 0 and form(n, torch.complex128, 19.0, False) == walk
+        assert (form(n, torch.float64, 40.0, False) == 0) == (n > 1) and form(n, torch.float64, 39.0, False) == walk
+        assert (form(n, torch.float64, 100.0, True) == 0) == (n == 3)
+        for dtype in (torch.complex64, torch.float32, torch.bfloat16):
+            assert (form(n, dtype, 100.0, False) == 0) == (n == 3)
+        assert form(n, torch.float32, 100.0, True) == walk
+    st = _plan.MatrixStats(20000, 20000, 1200000, 90, 60.0, 8.0, 0)
+    assert _plan.default_spmm_plan(st, 2, torch.float64).flags == 0
+    assert _plan.default_spmm_plan(st, 32, torch.float64).flags == walk
+    assert _plan.default_spmm_plan(st, 32, torch.bfloat16, acc_mode=nat.ACC_COMP).flags == 0
+
+
 def test_batch_stacking_is_block_diagonal():
     from flagsparse_public_b200 import batched, synthetic
     mats = [synthetic.poisson_uniform(r, c, mean=m, seed=s, device="cpu")
