@@ -319,11 +319,6 @@ def spmv_merge_items(n_rows, nnz):
     return _pow2_clamp((n_rows + nnz) / (SM_COUNT * 16), SPMV_MERGE_THREADS, 1024)
 
 
-def rows_skewed(max_row, mean):
-    """Whether a few rows dominate: the longest above 8 times the mean + 256."""
-    return max_row > 8 * max(mean, 1.0) + 256
-
-
 def default_spmv_plan(stats, dtype, row_cap=0, index_bytes=4):
     """Heuristic SpMV plan: merge path for skewed rows that are short on
     average (or of medium length in a large matrix or beside a very long row),
@@ -354,12 +349,29 @@ def seq_items_per_unit(stats):
 WALK_WARPS_PER_SM = 24  # resident warps of the range-walk SpMM kernel (6 CTAs of 4)
 
 
-def walk_items_per_unit(n_rows, nnz):
-    """Merge-path unit size for the range-walk SpMM kernel: one wave of its
-    resident warps, between 128 and 1024 items (power-law matrix, N = 64: 128
-    items 105 us, 256 88, 512 85, 1024 81; 100000 rows of 4, N = 32: 128 and
-    256 items 20 us, 512 24)."""
-    return _pow2_clamp((int(n_rows) + int(nnz)) / (SM_COUNT * WALK_WARPS_PER_SM), 128, 1024)
+def walk_items_per_unit(n_rows, nnz, n_dense):
+    """Merge-path unit size of the selector's range-walk plans: of 128, 256, 512
+    and 1024 items the one with the least (whole waves of resident warps) x
+    (items + a unit's own cost: 320 items up to 16 columns, 128 up to 32, 96
+    beyond, twice that for rows of 64 nonzeros or more, which more units split).
+    Unit counts just above a wave are what costs: 2.5 M items 512 per unit 1.1 x
+    the time of 1024, 4.5 M items 1024 per unit 1.03 - 1.17 x the time of 512
+    from 16 columns on (rows below 64).  2000 seeded matrices of five families
+    (10^4 to 2 * 10^6 rows, means of 2 to 128, float32), time over the best of
+    the four, geometric mean at 1 / 8 / 16 / 32 / 64 / 128 columns: this rule
+    1.013 / 1.011 / 1.012 / 1.008 / 1.010 / 1.012; the power of two next to
+    (rows + nonzeros) over 24 warps per SM 1.024 / 1.027 / 1.027 / 1.030 / 1.042
+    / 1.051, over 64 (seq_items_per_unit, which products without a selector pass
+    use) 1.078 / 1.064 / 1.058 / 1.051 / 1.039 / 1.033."""
+    n_rows, nnz = int(n_rows), int(nnz)
+    own = (320 if n_dense <= 16 else 128 if n_dense <= 32 else 96) * (2 if nnz >= 64 * n_rows else 1)
+    tiles = -(-max(int(n_dense), 1) // 128)
+
+    def cost(items):
+        units = -(-(n_rows + nnz) // items)
+        return -(-units * tiles // (SM_COUNT * WALK_WARPS_PER_SM)) * (items + own)
+
+    return min((128, 256, 512, 1024), key=cost)
 
 
 def spmm_form(n_dense, dtype, mean, skewed):
@@ -380,6 +392,11 @@ def spmm_form(n_dense, dtype, mean, skewed):
     if dtype == torch.complex128 or (n_dense == 3 and (dtype.itemsize >= 8 or not skewed)):
         return 0
     return 0 if dtype == torch.float64 and n_dense > 1 and not skewed else nat.PLAN_WALK
+
+
+def rows_skewed(max_row, mean):
+    """Whether a few rows dominate: the longest above 8 times the mean + 256."""
+    return max_row > 8 * max(mean, 1.0) + 256
 
 
 def fit_form(plan, row_ptr, n_rows, nnz, n_dense, dtype):

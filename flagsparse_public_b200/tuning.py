@@ -277,29 +277,51 @@ def targets_from_times(times):
 
 
 # ---------------------------------------------------------------- selector
-# Row-group picks stay below this many path items (rows + nonzeros); above it
-# the range-walk kernel is the faster one.  Measured on 200 held-out (matrix,
-# N) pairs with a row-group pick, walk time over row-group time: 1.2 - 1.3 at
-# 10^4 rows (launch bound), 1.0 at 0.5 - 1.5 M items, 0.87 at 2 - 10 M, 0.63 -
-# 0.8 above.
+# Row-group picks stay below this many path items (rows + nonzeros), twice as
+# many for rows of 32 nonzeros or more, and below 2^24 / N of them at N columns.
 ROW_GROUP_MAX_ITEMS = 1 << 20
+ROW_GROUP_MAX_ELEMENTS = 1 << 24
 
 
-def fit_to_walk(plan, n_rows, nnz, acc_mode):
-    """The selector's CUDA-core pick in the range-walk kernel's terms.  The
-    network's candidates were timed with the earlier merge-path form, whose
-    best units were smaller: a merge-path pick keeps its column tile and takes
-    its unit size from ``walk_items_per_unit`` (held-out power-law matrices:
-    1.12 x the best candidate with the pick's own units, 1.06 x with these),
-    and a large row-group or plain merge pick becomes the range walk.
-    Compensated sums run in the earlier form and keep the pick."""
+def keeps_row_groups(n_rows, nnz, n_dense, value_bytes):
+    """Whether a row-group pick of the selector runs as it is (else as the
+    range walk).  Row groups over range-walk time, geometric mean over the
+    picks on 2000 seeded matrices: below 10^6 items 0.71 - 0.92 at 1, 8 and 16
+    columns, above 0.9 - 2.0; rows of 32 or more at 1 - 2 * 10^6 items 0.76 -
+    0.95; 32 columns 0.71 - 0.95 below 6 * 10^5 items, 1.0 - 1.8 above; 64
+    columns 0.75 - 0.88 below 3 * 10^5, 1.0 - 1.8 above; 128 columns 0.70 - 0.77
+    below 10^5, 0.96 - 1.5 above.  Rows of 64 or more up to 8 * 10^6 items stay
+    ahead in float32 at 1 (0.84 - 0.94), 8 (0.81 - 0.87) and 16 columns (0.76 -
+    0.81), and in every type at 3 (0.8); not at other narrow widths, whose lane
+    vectors or scalars leave lanes idle (20000 rows of 400: 7 columns 89 us for
+    64, bfloat16 2 / 4 / 8 columns 52 / 72 / 73 us for 41 / 55 / 60)."""
+    items, mean = n_rows + nnz, nnz / max(n_rows, 1)
+    limit = ROW_GROUP_MAX_ITEMS * (2 if mean >= 32.0 else 1)
+    if items < min(limit, ROW_GROUP_MAX_ELEMENTS / n_dense):
+        return True
+    return mean >= 64.0 and items < 1 << 23 and (n_dense == 3 or (value_bytes >= 4 and n_dense in (1, 8, 16)))
+
+
+def fit_to_walk(plan, n_rows, nnz, n_dense, value_bytes, acc_mode, form=nat.PLAN_WALK):
+    """The selector's CUDA-core pick in the present kernels' terms.  The
+    network's candidates were timed with k_spmm_seq, which was slower than the
+    range walk and had its best units elsewhere: a merge-path pick keeps its
+    column tile and takes its unit size from ``walk_items_per_unit``, and
+    row-group and plain merge picks become the range walk where that is faster
+    (``keeps_row_groups``).  ``form``: spmm_form of the call; the few calls
+    that k_spmm_seq runs faster keep the pick's own units.  Compensated sums
+    run in k_spmm_seq and keep the pick."""
     if acc_mode == nat.ACC_COMP or isinstance(plan, _plan.BsrPlan):
         return plan
-    items = _plan.walk_items_per_unit(n_rows, nnz)
+    items = _plan.walk_items_per_unit(n_rows, nnz, n_dense)
     if plan.flags & nat.PLAN_WALK:
-        plan.items_per_unit = items
-    elif n_rows + nnz >= ROW_GROUP_MAX_ITEMS:
-        return _seq(items)()
+        if form:
+            plan.items_per_unit = items
+        else:
+            plan.flags &= ~nat.PLAN_WALK
+    elif plan.algo != nat.ALGO_ROWS or not keeps_row_groups(n_rows, nnz, n_dense, value_bytes):
+        plan = _seq(items)()
+        plan.flags = form
     return plan
 
 
@@ -356,11 +378,15 @@ class LearnedSelector:
                 feasible[BSR_CANDIDATE] = False
                 k, confident = self.choose(f, feasible)
             else:
-                self.last = ("learned", CANDIDATE_NAMES[k])
+                self.last = ("learned", plan.describe())
                 return plan
         if confident:
-            self.last = ("learned", CANDIDATE_NAMES[k])
-            return fit_to_walk(SPMM_CANDIDATES[k][1](), int(n_rows), int(data.numel()), acc_mode)
+            n_rows, nnz, n_dense = int(n_rows), int(data.numel()), int(B.shape[1])
+            mean = nnz / max(n_rows, 1)
+            form = _plan.spmm_form(n_dense, data.dtype, mean, _plan.rows_skewed(2 ** f[5] - 1, mean))
+            plan = fit_to_walk(SPMM_CANDIDATES[k][1](), n_rows, nnz, n_dense, data.element_size(), acc_mode, form)
+            self.last = ("learned", plan.describe())
+            return plan
         plan, _ = self.autotuner.tune(data, indices, indptr, n_rows, n_cols, B, C, acc_mode)
         self.last = ("autotune", plan.describe())
         return plan
@@ -462,14 +488,31 @@ def selectable(features, times):
     return ok
 
 
+def _figures(features):
+    """(rows, nonzeros, columns) of a raw feature vector."""
+    return int(round(2 ** features[0])) - 1, int(round(2 ** features[2])) - 1, int(round(2 ** features[10]))
+
+
 def heuristic_choice(features):
     """Candidate index the default heuristic (no selector) would run: the
-    batched merge-path kernel with the unit size of seq_items_per_unit."""
-    n_rows = 2 ** features[0] - 1
-    nnz = 2 ** features[2] - 1
-    st = _plan.MatrixStats(int(n_rows), 0, int(nnz), 0, nnz / max(n_rows, 1), 0.0, 0)
-    items = _plan.seq_items_per_unit(st)
-    return CANDIDATE_NAMES.index(f"seq{items}")
+    range walk with the unit size of seq_items_per_unit."""
+    n_rows, nnz, _ = _figures(features)
+    st = _plan.MatrixStats(n_rows, 0, nnz, 0, nnz / max(n_rows, 1), 0.0, 0)
+    return CANDIDATE_NAMES.index(f"seq{_plan.seq_items_per_unit(st)}")
+
+
+def fitted_choice(features, choice):
+    """Candidate index that runs for a pick of the network (fit_to_walk), for
+    scoring on the times of the present kernels: the candidate with the fitted
+    plan's parameters (a tiled pick, of which only two unit sizes are timed,
+    the nearer one)."""
+    if choice == BSR_CANDIDATE:
+        return choice
+    plan = fit_to_walk(SPMM_CANDIDATES[choice][1](), *_figures(features), int(features[14] * 8), nat.ACC_NATIVE)
+    if plan.flags & nat.PLAN_WALK and plan.n_tile:
+        return CANDIDATE_NAMES.index("seq1024_t32" if plan.items_per_unit >= 512 else "seq256_t32")
+    keys = [make().key() if make is not _plan.BsrPlan else None for _, make in SPMM_CANDIDATES]
+    return keys.index(plan.key())
 
 
 def regret(times, choice):
@@ -531,6 +574,7 @@ def main(argv=None):
             continue
         pred = mlp.forward(to(X[sel])).cpu().numpy()
         learned = np.argmin(np.where(selectable(F[sel], Tm[sel]), pred, np.inf), axis=1)
+        learned = np.asarray([fitted_choice(f, k) for f, k in zip(F[sel], learned)])
         heur = np.asarray([heuristic_choice(f) for f in F[sel]])
         r_learned = regret(Tm[sel], learned)
         r_heur = regret(Tm[sel], heur)

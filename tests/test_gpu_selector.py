@@ -187,3 +187,15 @@ def test_bsr_candidate_runs_through_run_spmm():
     Bs = synthetic.dense_operand(sc, 32, seed=8, dtype=torch.bfloat16, device=DEV)
     with pytest.raises(ValueError, match="fill-in"):
         _plan.run_spmm(sd, si, sp, sr, sc, Bs, torch.empty((sr, 32), device=DEV), nat.ACC_NATIVE, _plan.BsrPlan())
+
+
+def test_last_describes_the_plan_that_runs():
+    """A large row-group pick runs as the range walk, and says so."""
+    sel = tuning.LearnedSelector()
+    for rows, mean in ((20000, 8.0), (400000, 8.0)):
+        data, indices, indptr, (n_rows, n_cols) = synthetic.poisson_uniform(rows, rows, mean=mean, seed=9, device=DEV)
+        for n_dense in (1, 8, 32):
+            B = synthetic.dense_operand(n_cols, n_dense, seed=1, device=DEV)
+            C = torch.empty((n_rows, n_dense), device=DEV)
+            plan = sel.select(data, indices, indptr, n_rows, n_cols, B, C, nat.ACC_NATIVE)
+            assert sel.last == ("learned", plan.describe())

@@ -226,6 +226,20 @@ def test_spmm_form_of_narrow_operands():
     assert _plan.default_spmm_plan(st, 32, torch.bfloat16, acc_mode=nat.ACC_COMP).flags == 0
 
 
+def test_walk_units():
+    """Units of whole waves of 148 x 24 warps; a unit's own cost keeps them
+    from getting small."""
+    wave = 148 * 24
+    for n in (1, 16, 32, 128):
+        assert [_plan.walk_items_per_unit(wave * i, 0, n) for i in (128, 256, 512, 1024)] == [128, 256, 512, 1024]
+        assert _plan.walk_items_per_unit(10 ** 9, 0, n) == 1024 and _plan.walk_items_per_unit(1, 0, n) == 128
+    # 1.3 waves of 1024: two whole ones of 1024 or three of 512
+    assert _plan.walk_items_per_unit(wave * 1330, 0, 32) == 512
+    # rows of 64 or more: twice a unit's own cost
+    assert _plan.walk_items_per_unit(wave * 20, wave * 1260, 16) == 512
+    assert _plan.walk_items_per_unit(wave * 10, wave * 1270, 16) == 1024
+
+
 def test_batch_stacking_is_block_diagonal():
     from flagsparse_public_b200 import batched, synthetic
     mats = [synthetic.poisson_uniform(r, c, mean=m, seed=s, device="cpu")

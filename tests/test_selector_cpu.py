@@ -5,7 +5,8 @@ import math
 import numpy as np
 import pytest
 
-from flagsparse_public_b200 import tuning
+from flagsparse_public_b200 import _native as nat
+from flagsparse_public_b200 import _plan, tuning
 from oracle import mlp as omlp
 
 
@@ -150,3 +151,62 @@ def test_selector_fallback_triggers_outside_training_range():
     w = np.load(tuning.WEIGHTS_PATH, allow_pickle=False)
     z_far = np.abs((np.full(tuning.N_FEATURES, 1e3) - w["mu"]) / w["sigma"])
     assert np.any(z_far > 4.0)
+
+
+def test_fit_to_walk():
+    """A pick in the present kernels' terms: merge-path picks take the range
+    walk's unit and keep their column tile, row groups stay where they are the
+    faster ones, compensated sums and the BSR path keep the pick."""
+    cand = dict(tuning.SPMM_CANDIDATES)
+    small, large = (20000, 200000), (1000000, 8000000)
+    for name, tile in (("seq128", 0), ("seq1024", 0), ("seq256_t32", 32)):
+        p = tuning.fit_to_walk(cand[name](), *large, 64, 4, nat.ACC_NATIVE)
+        assert p.flags == nat.PLAN_WALK and p.n_tile == tile
+        assert p.items_per_unit == _plan.walk_items_per_unit(*large, 64)
+        assert tuning.fit_to_walk(cand[name](), *large, 64, 4, nat.ACC_COMP).key() == cand[name]().key()
+    for name in ("vector_rows", "rows8", "warp_rows", "warp_rows_t32"):
+        assert tuning.fit_to_walk(cand[name](), *small, 32, 4, nat.ACC_NATIVE).key() == cand[name]().key()
+        p = tuning.fit_to_walk(cand[name](), *large, 8, 4, nat.ACC_NATIVE)
+        assert p.algo == nat.ALGO_SEQ and p.flags == nat.PLAN_WALK and p.n_tile == 0
+    assert tuning.fit_to_walk(cand["merge128"](), *small, 8, 4, nat.ACC_NATIVE).algo == nat.ALGO_SEQ
+    assert isinstance(tuning.fit_to_walk(cand["bsr16_tc"](), *large, 64, 2, nat.ACC_NATIVE), _plan.BsrPlan)
+    # a call that k_spmm_seq runs faster keeps the pick's units
+    p = tuning.fit_to_walk(cand["seq128"](), 20000, 1200000, 3, 4, nat.ACC_NATIVE, form=0)
+    assert p.flags == 0 and p.items_per_unit == 128
+
+
+@pytest.mark.parametrize("rows,mean,n_dense,value_bytes,keeps", [
+    (100000, 8, 8, 4, True), (200000, 8, 8, 4, False),  # 2^20 items
+    (40000, 32, 1, 4, True), (70000, 32, 1, 4, False),  # 2^21 from rows of 32 on
+    (50000, 9, 32, 4, True), (60000, 9, 32, 4, False),  # 2^24 / N items
+    (12000, 9, 128, 4, True), (20000, 9, 128, 4, False),
+    (50000, 100, 1, 4, True), (50000, 100, 16, 4, True), (50000, 100, 3, 2, True),  # long rows
+    (50000, 100, 8, 2, False), (50000, 100, 2, 4, False), (50000, 100, 7, 4, False), (50000, 100, 17, 4, False),
+    (50000, 63, 8, 4, False), (90000, 100, 8, 4, False)])
+def test_row_group_picks_stay_where_they_win(rows, mean, n_dense, value_bytes, keeps):
+    assert tuning.keeps_row_groups(rows, rows * mean, n_dense, value_bytes) == keeps
+
+
+def test_fitted_picks_on_the_present_kernels():
+    """The plans that run (the network's picks after fit_to_walk) against the
+    times of the present kernels for the same held-out samples (8 timed calls
+    per candidate on a B200; candidates in the range-walk form): within 5 % of
+    exhaustive autotuning on the 400 corpus matrices, within 7 % on the 40
+    larger ones, closer than the picks as they are and than the heuristic."""
+    import os
+    from tests.conftest import GOLDEN_DIR
+    F, _, _, kind = _heldout()
+    z = np.load(os.path.join(GOLDEN_DIR, "selector_heldout_walk_times.npz"), allow_pickle=False)
+    assert tuple(str(s) for s in z["names"]) == tuning.CANDIDATE_NAMES
+    times = z["times"].astype(np.float64)
+    w = np.load(tuning.WEIGHTS_PATH, allow_pickle=False)
+    pred, _ = omlp.forward((F - w["mu"]) / w["sigma"], w["params"].astype(np.float64), tuple(int(v) for v in w["dims"]))
+    picks = np.argmin(np.where(tuning.selectable(F, times), pred, np.inf), axis=1)
+    fitted = np.asarray([tuning.fitted_choice(f, k) for f, k in zip(F, picks)])
+    heur = np.asarray([tuning.heuristic_choice(f) for f in F])
+    best = np.where(np.isfinite(times), times, np.inf).min(axis=1)
+    for slice_kind, bound in ((1, 1.05), (2, 1.07)):
+        s = kind == slice_kind
+        total = {name: times[s, c[s]].sum() / best[s].sum() for name, c in
+                 (("picks", picks), ("fitted", fitted), ("heuristic", heur))}
+        assert total["fitted"] <= bound and total["fitted"] < min(total["picks"], total["heuristic"]), total
