@@ -47,6 +47,7 @@ class PreparedCsrSpmmOptAlg2:
         "supports_opt",
         "_stats",
         "_plans",
+        "_one_shot",
     )
 
     def __init__(self, data, kernel_indices, kernel_indptr, shape, n_rows, n_cols, row_lengths, max_row_nnz,
@@ -63,6 +64,7 @@ class PreparedCsrSpmmOptAlg2:
         self.supports_opt = data.dtype in SUPPORTED_SPMM_OPT_ALG2_DTYPES
         self._stats = None
         self._plans = {}
+        self._one_shot = False
 
 
 def _normalize_spmm_opt_alg2_device_props(device):
@@ -96,14 +98,15 @@ def _build_spmm_opt_alg2_buckets(row_lengths, dtype):
 
 
 def prepare_spmm_csr_opt_alg2(data, indices, indptr, shape):
-    (data, kernel_indices, kernel_indptr, n_rows, n_cols, row_lengths, max_row_nnz) = _prepare_spmm_csr_matrix(
-        data, indices, indptr, shape
-    )
+    (data, kernel_indices, kernel_indptr, n_rows, n_cols, row_lengths, max_row_nnz,
+     stats) = _prepare_spmm_csr_matrix(data, indices, indptr, shape, return_stats=True)
     opt_buckets = _build_spmm_opt_alg2_buckets(row_lengths, data.dtype)
-    return PreparedCsrSpmmOptAlg2(
+    p = PreparedCsrSpmmOptAlg2(
         data=data, kernel_indices=kernel_indices, kernel_indptr=kernel_indptr, shape=shape, n_rows=n_rows,
         n_cols=n_cols, row_lengths=row_lengths, max_row_nnz=max_row_nnz, opt_buckets=opt_buckets,
     )
+    p._stats = stats
+    return p
 
 
 def _validate_spmm_opt_alg2_runtime_inputs(prepared, B, out):
@@ -169,6 +172,7 @@ def flagsparse_spmm_csr_opt_alg2(data=None, indices=None, indptr=None, B=None, s
         if any(arg is None for arg in (data, indices, indptr, shape)):
             raise ValueError("data, indices, indptr, and shape are required when prepared is not provided")
         prepared = prepare_spmm_csr_opt_alg2(data, indices, indptr, shape)
+        prepared._one_shot = True  # this object does not outlive the call
     elif shape is not None:
         resolved_shape = (int(shape[0]), int(shape[1]))
         if resolved_shape != prepared.shape:

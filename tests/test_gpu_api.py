@@ -616,3 +616,23 @@ def test_spmv_malformed_both_routes(kind, exc, msg, index_dtype):
     d, i, p, shape = _malformed(kind)
     with pytest.raises(exc, match=msg):
         fs.flagsparse_spmv_csr(d, i.to(index_dtype), p, torch.ones(3, device=DEV), shape)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_one_shot_alg2_skips_the_selector(dtype, monkeypatch):
+    """alg2 without a prepared object multiplies a matrix once: no selector
+    pass and no ticket set-up, as in flagsparse_spmm_csr_opt; a prepared object
+    still goes through the selector."""
+    from flagsparse_public_b200 import _plan, synthetic
+
+    d, i, p, shape = synthetic.zipf_powerlaw(3000, 3000, alpha=1.8, mean=12.0, cap=2000, seed=4, device=DEV)
+    d = d.to(dtype)
+    B = torch.randn(shape[1], 24, device=DEV, dtype=torch.float64).to(dtype)
+    prep = fs.prepare_spmm_csr_opt_alg2(d, i, p, shape)
+    ref = fs.flagsparse_spmm_csr_opt_alg2(B=B, prepared=prep)
+    chosen = []
+    monkeypatch.setattr(_plan, "chosen_spmm_plan", lambda *a, **k: chosen.append(1))
+    C, meta = fs.flagsparse_spmm_csr_opt_alg2(d, i, p, B, shape, return_meta=True)
+    assert not chosen and len(meta["launch_configs"]) == 1
+    tol = 1e-4 if dtype == torch.float32 else 1e-11
+    torch.testing.assert_close(C, ref, rtol=tol, atol=tol)
