@@ -56,6 +56,18 @@ def test_complex32_all_plans(pattern, n_dense):
         _check(C, exact, mag)
 
 
+@pytest.mark.parametrize("pattern", ["empty_rows", "boundaries", "skewed", "one_row"])
+@pytest.mark.parametrize("n_dense", [1, 3, 8, 33, 64])
+def test_complex32_range_walk(pattern, n_dense):
+    lengths = EDGE_LENGTHS[pattern][::3] if pattern == "skewed" else EDGE_LENGTHS[pattern]
+    data, indices, indptr, n_rows, n_cols, B, exact, mag = _case(lengths, 13000, n_dense, 62)
+    for items, snap in ((128, 0), (1024, 64)):
+        C = torch.empty((n_rows, n_dense), dtype=C32, device=DEV)
+        _plan.run_spmm(data.to(DEV), indices.to(DEV), indptr.to(DEV), n_rows, n_cols, B.to(DEV), C, nat.ACC_NATIVE,
+                       _plan.KernelPlan(nat.ALGO_SEQ, items_per_unit=items, snap=snap, flags=nat.PLAN_WALK))
+        _check(C, exact, mag)
+
+
 def test_complex32_public_csr_and_coo():
     lengths = [5, 0, 40, 7, 300, 1, 0, 2000, 3]
     data, indices, indptr, n_rows, n_cols, B, exact, mag = _case(lengths, 5000, 24, 63)

@@ -88,6 +88,25 @@ def test_spmv_unaligned_views_use_scalar_path():
         assert scaled_error(y, exact, mag) <= 1e-5
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.float16, torch.complex64, torch.complex128])
+@pytest.mark.parametrize("index_dtype", [torch.int32, torch.int64])
+def test_spmv_merge_on_unaligned_views(dtype, index_dtype):
+    """Values or indices off the 16-byte grid: the merge path's single-element
+    loads, rows over several units and ragged ends included."""
+    data, indices, indptr, (n_rows, n_cols) = csr_from_lengths([5, 0, 9, 700, 33, 64, 3, 0, 1, 259], 800, seed=13,
+                                                               dtype=dtype, index_dtype=index_dtype)
+    x = dense((n_cols,), 14, dtype)
+    exact, mag = orc.spmv_csr_exact(data, indices, indptr, x)
+    for shift_data, shift_idx in ((1, 0), (0, 1), (1, 1)):
+        d = torch.cat([torch.zeros(shift_data, dtype=dtype), data]).to(DEV)[shift_data:]
+        i = torch.cat([torch.zeros(shift_idx, dtype=index_dtype), indices]).to(DEV)[shift_idx:]
+        for items in (128, 1024):
+            y = torch.full((n_rows,), float("nan"), dtype=dtype, device=DEV)
+            _plan.run_spmv(d, i, indptr.to(DEV), n_rows, n_cols, x.to(DEV), y, nat.ACC_NATIVE,
+                           _plan.KernelPlan(nat.ALGO_MERGE, items_per_unit=items))
+            assert scaled_error(y, exact, mag) <= max(REL_BOUND[dtype], 3e-5 if dtype == torch.float32 else 0.0)
+
+
 def test_spmv_row_cap_truncates_like_reference_window():
     data, indices, indptr, (n_rows, n_cols) = csr_from_lengths([10, 40, 70, 0, 33], 200, seed=11)
     x = dense((n_cols,), 12, torch.float32)

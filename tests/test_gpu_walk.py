@@ -2,11 +2,16 @@
 the FP64 oracle where it can go wrong: rows at the edges of batches (8), chunks
 (256), units and sub-group ranges, ranges without a nonzero, rows that end
 where a unit begins, runs of empty rows, and every lane layout (whole 16-byte
-lane vectors and strided columns of odd widths).
+lane vectors and strided columns: every compiled columns x lanes pair by a
+width that picks it), B and C with rows further apart than their width or off
+the 16-byte grid.
 
-Bounds (condition-scaled, tests/numerics.py): those of the other SpMM forms;
-n products summed in float32 err by at most about n * 2^-24 of their
-magnitude, 3e-5 for the longest row here (300 in a chain of 8 + 300 / 8)."""
+Bounds (condition-scaled, tests/numerics.py): those of the other SpMM forms.
+A float32 sum's chains are at most 4 products of a batch, 2 sums of pairs, the
+range's batches (at most 256 / 8 in a chunk) and the chunks: below 45
+additions for the longest row here (511), 45 * 2^-24 = 2.7e-6 of the magnitude
+and one rounding of the result, so 1e-5 holds with room; the 3e-5 of the
+float32 modes also covers one serial chain of 500."""
 
 import pytest
 import torch
@@ -34,6 +39,9 @@ MODES = [(torch.float32, nat.ACC_NATIVE, torch.float32, 3e-5),
          (torch.float32, nat.ACC_WIDE, torch.float32, REL_BOUND[torch.float32]),
          (torch.float64, nat.ACC_NATIVE, torch.float64, REL_BOUND[torch.float64]),
          (torch.bfloat16, nat.ACC_NATIVE, torch.float32, 3e-5),
+         (torch.float16, nat.ACC_NATIVE, torch.float32, 3e-5),
+         (torch.complex64, nat.ACC_NATIVE, torch.complex64, 3e-5),
+         (torch.complex64, nat.ACC_WIDE, torch.complex64, REL_BOUND[torch.complex64]),
          (torch.complex128, nat.ACC_NATIVE, torch.complex128, REL_BOUND[torch.complex128])]
 
 
@@ -50,7 +58,7 @@ def test_walk_matches_oracle(pattern, mode):
         PATTERNS[pattern], 600, seed=61, dtype=dtype, index_dtype=torch.int64 if wide_idx else torch.int32,
         ptr_dtype=torch.int32 if wide_idx else torch.int64)
     d = (data.to(DEV), indices.to(DEV), indptr.to(DEV))
-    for n_dense in (1, 3, 5, 16, 33, 40, 64, 100, 130):
+    for n_dense in (1, 2, 3, 5, 6, 9, 13, 16, 19, 33, 40, 51, 64, 67, 95, 100, 130):
         B = dense((n_cols, n_dense), 62, dtype)
         exact, mag = orc.spmm_csr_exact(data, indices, indptr, B)
         Bd = B.to(DEV)
@@ -82,6 +90,28 @@ def test_walk_leaves_non_finite_b_rows_alone():
     _plan.run_spmm(data.to(DEV), indices.to(DEV), indptr.to(DEV), n_rows, n_cols, B.to(DEV), C, nat.ACC_NATIVE,
                    _plan.KernelPlan(nat.ALGO_SEQ, items_per_unit=128, flags=nat.PLAN_WALK))
     assert scaled_error(C, exact, mag) <= 3e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.float16, torch.complex64])
+@pytest.mark.parametrize("view", ["pitch", "column", "row_pitch_odd"])
+def test_walk_on_views_of_b_and_c(dtype, view):
+    """B and C as column ranges of wider arrays: rows a multiple of 16 bytes
+    apart (lane vectors), the same starting off the 16-byte grid and an odd row
+    pitch (strided columns); columns beside C's stay as they were."""
+    data, indices, indptr, (n_rows, n_cols) = csr_from_lengths(PATTERNS["chunk_edges"], 600, seed=65, dtype=dtype)
+    first, pitch = {"pitch": (0, 80), "column": (1, 80), "row_pitch_odd": (0, 67)}[view]
+    out_dtype = torch.float32 if dtype == torch.float16 else dtype
+    for n_dense in (8, 64):
+        wide = dense((n_cols, pitch), 66, dtype)
+        B = wide[:, first:first + n_dense]
+        exact, mag = orc.spmm_csr_exact(data, indices, indptr, B.contiguous())
+        Cw = torch.full((n_rows, pitch), 7.0, dtype=out_dtype, device=DEV)
+        C = Cw[:, first:first + n_dense]
+        _plan.run_spmm(data.to(DEV), indices.to(DEV), indptr.to(DEV), n_rows, n_cols,
+                       wide.to(DEV)[:, first:first + n_dense], C, nat.ACC_NATIVE,
+                       _plan.KernelPlan(nat.ALGO_SEQ, items_per_unit=256, snap=64, flags=nat.PLAN_WALK))
+        assert scaled_error(C, exact, mag) <= (REL_BOUND[dtype] if dtype == torch.float64 else 3e-5)
+        assert bool((Cw[:, :first] == 7).all()) and bool((Cw[:, first + n_dense:] == 7).all())
 
 
 @pytest.mark.parametrize("dtype,n_dense,mean", [(torch.complex128, 1, 400), (torch.complex128, 4, 60),
