@@ -505,34 +505,26 @@ extern "C" int fsb_spmm_csr(const fsb_csr* A, const void* B, int64_t ldb, int64_
     if (plan->algo == FSB_ALGO_GATHER)
         return spmm_gather_dispatch(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes,
                                     st);
-    if (plan->algo == FSB_ALGO_SEQ && (plan->flags & FSB_PLAN_WALK) && !(plan->flags & FSB_PLAN_TMA_GATHER) &&
-        walk_takes(A, ldb, ldc, out_dtype, acc_mode)) {
-        switch (A->value_dtype) {
-        case FSB_F16: return walk_dispatch_f16(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_BF16: return walk_dispatch_bf16(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_F32: return walk_dispatch_f32(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_F64: return walk_dispatch_f64(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_C32: return walk_dispatch_c32(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_C64: return walk_dispatch_c64(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_C128: return walk_dispatch_c128(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        default:
-            fsb_host::set_error("fsb_spmm_csr: value dtype code %d", A->value_dtype);
-            return FSB_ERR_UNSUPPORTED;
-        }
-    }
     if (plan->algo == FSB_ALGO_SEQ) {
+        const bool walk = (plan->flags & FSB_PLAN_WALK) && !(plan->flags & FSB_PLAN_TMA_GATHER) &&
+                          walk_takes(A, ldb, ldc, out_dtype, acc_mode);
+#define FSB_SEQ_CASE(CODE, T)                                                                                       \
+    case CODE:                                                                                                      \
+        return (walk ? walk_dispatch_##T : seq_dispatch_##T)(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, \
+                                                             workspace, workspace_bytes, st);
         switch (A->value_dtype) {
-        case FSB_F16: return seq_dispatch_f16(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_BF16: return seq_dispatch_bf16(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_F32: return seq_dispatch_f32(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_F64: return seq_dispatch_f64(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_C32: return seq_dispatch_c32(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_C64: return seq_dispatch_c64(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
-        case FSB_C128: return seq_dispatch_c128(A, B, ldb, n_dense, C, ldc, out_dtype, acc_mode, plan, workspace, workspace_bytes, st);
+            FSB_SEQ_CASE(FSB_F16, f16)
+            FSB_SEQ_CASE(FSB_BF16, bf16)
+            FSB_SEQ_CASE(FSB_F32, f32)
+            FSB_SEQ_CASE(FSB_F64, f64)
+            FSB_SEQ_CASE(FSB_C32, c32)
+            FSB_SEQ_CASE(FSB_C64, c64)
+            FSB_SEQ_CASE(FSB_C128, c128)
         default:
             fsb_host::set_error("fsb_spmm_csr: value dtype code %d", A->value_dtype);
             return FSB_ERR_UNSUPPORTED;
         }
+#undef FSB_SEQ_CASE
     }
     return dispatch_vao(A->value_dtype, acc_mode, out_dtype, [&](auto tv, auto ta, auto to) -> int {
         using V = typename decltype(tv)::type;

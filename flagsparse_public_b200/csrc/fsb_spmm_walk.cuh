@@ -1,6 +1,7 @@
 // fsb_spmm_walk.cuh -- the range-walk form of the batched merge-path SpMM
 // (FSB_ALGO_SEQ with FSB_PLAN_WALK; instantiated per value type in
-// fsb_spmm_walk_*.cu), the form the heuristics, the selector and the batch use.
+// fsb_spmm_walk_*.cu), the form the heuristics, the selector and the batch use
+// for all but narrow operands with long rows (spmm_form in _plan.py).
 //
 // One warp per (merge-path unit, column tile), as in fsb_spmm_seq.cuh.  The
 // unit's nonzeros pass through shared memory in chunks of kWalkChunk: columns,
@@ -11,7 +12,7 @@
 // stores its rows itself where their bits say so: no reduction across the warp
 // per row and no replay of a batch per row, which is what k_spmm_seq spends
 // most of its instructions on when rows are short (26 warp instructions per
-// nonzero on the power-law matrix at N = 64; 11 here).  Sub-groups meet once
+// nonzero on the power-law matrix at N = 64; 10 here).  Sub-groups meet once
 // per chunk, in a segmented scan of their open partials; a range's first row,
 // begun before the range, waits for that in shared memory.  Sums are
 // deterministic: batches of U, rows in order, sub-groups in order, units in
@@ -108,7 +109,7 @@ k_spmm_walk(const V* __restrict__ val, const I* __restrict__ col, const void* __
             int* __restrict__ tickets) {
     constexpr int LPN = 1 << LPN_LOG2;
     constexpr int NPAR = 32 >> LPN_LOG2;
-        constexpr int U = VW * (int)sizeof(V) * 8 <= 192 ? 8 : 4;  // B loads in flight per lane
+    constexpr int U = VW * (int)sizeof(V) * 8 <= 192 ? 8 : 4;  // B loads in flight per lane
     constexpr int CH = kWalkChunk;
     constexpr int WORDS = CH / 32;
     constexpr int kWarps = kSpmmThreads / 32;
@@ -118,7 +119,7 @@ k_spmm_walk(const V* __restrict__ val, const I* __restrict__ col, const void* __
     __shared__ __align__(16) V sm_val[kWarps][CH];
     __shared__ __align__(16) uint32_t sm_brk[kWarps][WORDS];  // bit per nonzero: a row starts here
     __shared__ __align__(16) A sm_head[kSpmmThreads][VW];  // a range's first row, finished before its part from earlier
-    __shared__ __align__(16) A sm_open[kSpmmThreads][VW];  // the open row's sum before the chunk (first sub-group's lanes)
+    __shared__ __align__(16) A sm_open[kSpmmThreads][VW];  // the open row's sum before the chunk (first sub-group)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t* s_col = sm_col[warp];
     int* s_row = sm_row[warp];
@@ -444,7 +445,8 @@ k_spmm_walk(const V* __restrict__ val, const I* __restrict__ col, const void* __
 
 template <class V, class A, class O, class I, int VW, bool STRIDED, int LPN_LOG2>
 void launch_walk_one(dim3 g, cudaStream_t st, const V* val, const I* col, const void* ptr, int ptr64, const V* B,
-                     uint32_t ldb_bytes, O* C, uint32_t ldc_bytes, int64_t n_rows, int64_t n_dense, const int64_t* coords, int64_t n_units, int64_t* carry_row, A* cv, A* hv, const int64_t* runs,
+                     uint32_t ldb_bytes, O* C, uint32_t ldc_bytes, int64_t n_rows, int64_t n_dense,
+                     const int64_t* coords, int64_t n_units, int64_t* carry_row, A* cv, A* hv, const int64_t* runs,
                      int* tickets) {
     k_spmm_walk<V, A, O, I, VW, LPN_LOG2, STRIDED><<<g, kSpmmThreads, 0, st>>>(
         val, col, ptr, ptr64, B, ldb_bytes, C, ldc_bytes, n_rows, n_dense, coords, n_units, carry_row, cv, hv, runs,
@@ -475,7 +477,7 @@ inline WalkTile walk_strided_tile(int64_t target) {
 }
 
 // Compiled accumulator / value pairs of this form: all but the compensated
-// ones.  FSB_ERR_UNSUPPORTED sends the call to k_spmm_seq.
+// ones (walk_takes keeps those calls in k_spmm_seq).
 template <class V, class A, class O, class I>
 int launch_walk(const fsb_csr* Am, const V* val, const I* col, const V* B, int64_t ldb, int64_t n_dense,
                 O* C, int64_t ldc, const fsb_plan* plan, void* workspace, int64_t workspace_bytes,
@@ -527,7 +529,8 @@ int launch_walk(const fsb_csr* Am, const V* val, const I* col, const V* B, int64
                                              runs, tickets);                                                         \
         done = true;                                                                                                 \
     }
-#define FSB_WALK6(W, S) FSB_WALK(W, 0, S) FSB_WALK(W, 1, S) FSB_WALK(W, 2, S) FSB_WALK(W, 3, S) FSB_WALK(W, 4, S) FSB_WALK(W, 5, S)
+#define FSB_WALK6(W, S)                                                                                          \
+    FSB_WALK(W, 0, S) FSB_WALK(W, 1, S) FSB_WALK(W, 2, S) FSB_WALK(W, 3, S) FSB_WALK(W, 4, S) FSB_WALK(W, 5, S)
     if constexpr (kMaxVW > 1) {
         FSB_WALK6(kMaxVW, false)
     }
@@ -581,8 +584,8 @@ int walk_dispatch_for(const fsb_csr* A, const void* B, int64_t ldb, int64_t n_de
                     return FSB_ERR_UNSUPPORTED;
                 }
                 return launch_walk<V, Ac, O, I>(A, static_cast<const V*>(A->values), static_cast<const I*>(A->col_idx),
-                                                static_cast<const V*>(B), ldb, n_dense, static_cast<O*>(C), ldc, plan, workspace, workspace_bytes,
-                                                st);
+                                                static_cast<const V*>(B), ldb, n_dense, static_cast<O*>(C), ldc, plan,
+                                                workspace, workspace_bytes, st);
             });
         }
     });

@@ -1,10 +1,12 @@
 // fsb_spmv.cu -- CSR SpMV on sm_100a: y = A x.
 //
 // Two kernel families, chosen per matrix by the host plan:
-//   * k_spmv_rows  : a group of 2^k lanes per row (k = 0..5; 32 lanes is
-//                    warp-per-row), 128-bit streaming loads of values and column
-//                    indices on the aligned body of each row, read-only cached
+//   * k_spmv_rows  : a group of 2^k lanes per row (k = 0..5), 128-bit streaming
+//                    loads of values and column indices, read-only cached
 //                    gathers of x, xor-butterfly reduction inside the group.
+//                    Up to 16 lanes take the aligned chunks that cover the row,
+//                    the elements outside it masked; a whole warp per row takes
+//                    the aligned body and single elements at its two ends.
 //   * k_spmv_merge : merge-path units of equal (row ends + nonzeros) whatever
 //                    the row-length skew (Merrill & Garland, SC'16), a warp per
 //                    unit.  Each lane sums 8 consecutive nonzeros in order and
@@ -118,8 +120,8 @@ __device__ __forceinline__ A row_partial(const V* __restrict__ val, const I* __r
 // 355 and 451, bfloat16 232 and 304).
 template <class V, class A, class I>
 __device__ __forceinline__ A row_partial_wide(const V* __restrict__ val, const I* __restrict__ col,
-                                         const V* __restrict__ x, int64_t s, int64_t e,
-                                         int lane, int T, bool vec_ok) {
+                                              const V* __restrict__ x, int64_t s, int64_t e,
+                                              int lane, int T, bool vec_ok) {
     constexpr int VV = VecWidth<V>::value;
     constexpr int VI = VecWidth<I>::value;
     constexpr int VEC = VV < VI ? VV : VI;
@@ -216,6 +218,7 @@ k_spmv_rows(const V* __restrict__ val, const I* __restrict__ col, const P* __res
 // the next chunk's columns and row offsets a chunk ahead: 150 us (float64).
 // 8 resident CTAs (64 registers) for values below 8 bytes, 6 (80) else: 173 us
 // with 8 for float64.
+
 // N consecutive elements from an address that is a multiple of 16 bytes (or of
 // the N elements where those are fewer bytes), in streaming vector loads.
 template <class T, int N>
@@ -593,9 +596,14 @@ extern "C" int fsb_spmv_csr(const fsb_csr* A, const void* x, void* y, int out_dt
 namespace {
 int64_t check_bytes(const fsb_csr* A) { return align_up(fsb_csr_check_workspace_bytes(A->n_rows, A->nnz), 256); }
 
-// Lanes of a row group.  `chunk` is the elements of one 16-byte step of a lane
-// (spmv_chunk: the smaller of the value and the index vector); a lane should have a few
-// whole steps of its row, and a row of hundreds of nonzeros a whole warp:
+// Elements of one 16-byte step of a lane: the smaller of the value and the
+// index vector.
+int spmv_chunk(int value_bytes, int index_bytes) {
+    return 16 / std::max(1, std::min(16, std::max(value_bytes, index_bytes)));
+}
+
+// Lanes of a row group: a lane should have a few whole steps of `chunk`
+// elements of its row, and a row of hundreds of nonzeros a whole warp:
 //   chunk 4 (32-bit indices, values up to 4 bytes): 2 lanes, 4 from 12 (24
 //           where the rows alone fill the chip) nonzeros on average, 8 from
 //           80, 16 from 200, 32 from 512;
@@ -619,10 +627,6 @@ int64_t check_bytes(const fsb_csr* A) { return align_up(fsb_csr_check_workspace_
 // indices: 50 us, 25 with 32 lanes).
 // Rows that a few long ones dominate (skewed, off the merge path) take a whole
 // warp.  default_spmv_plan in _plan.py follows the same rule.
-int spmv_chunk(int value_bytes, int index_bytes) {
-    return 16 / std::max(1, std::min(16, std::max(value_bytes, index_bytes)));
-}
-
 int spmv_row_lanes(int64_t n_rows, double mean, int chunk, bool skewed) {
     if (skewed) return 32;
     int lanes;

@@ -94,8 +94,9 @@ extern "C" {
                                   contiguous part of the unit's nonzeros (staged
                                   in shared memory with their rows) and stores
                                   its rows itself; calls it does not take
-                                  (compensated accumulators, more than 2^32
-                                  columns) run in the plain SEQ form          */
+                                  (compensated accumulators, a row_map, 2^32
+                                  columns or more, rows of B or C 2^32 bytes
+                                  apart or more) run in the plain SEQ form    */
 
 /* A CSR matrix (or a sorted COO matrix seen as row runs).
  * row_ptr has n_rows + 1 entries.  If row_map is non-null, row r of this
