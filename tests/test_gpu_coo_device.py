@@ -138,3 +138,23 @@ def test_coo_spmv_sizes_need_no_host_read():
     eager = fs.flagsparse_spmv_coo(vals, row, col, x, (50000, 50000))
     _gr, y = _capture(lambda: fs.flagsparse_spmv_coo(vals, row, col, x, (50000, 50000)))
     assert torch.equal(y, eager)
+
+
+@pytest.mark.parametrize("mean", [2, 60])
+def test_coo_spmv_writes_every_row(mean):
+    """The run route allocates y without clearing it: rows without entries, at
+    the ends and between, come out zero whatever the memory held."""
+    g = torch.Generator(device=DEV).manual_seed(mean)
+    n = 3000
+    row = torch.randint(100, n - 200, (n * mean,), generator=g, device=DEV)
+    row += row % 2  # odd rows stay empty
+    col = torch.randint(0, n, (n * mean,), generator=g, device=DEV)
+    data, x = torch.rand(n * mean, generator=g, device=DEV), torch.rand(n, generator=g, device=DEV)
+    prepared = fs.prepare_spmv_coo(data, row, col, (n, n))
+    ref = torch.zeros(n, dtype=torch.float64, device=DEV).index_add_(0, row, data.double() * x[col].double())
+    for _ in range(3):
+        held = [torch.full((n,), float("nan"), device=DEV) for _ in range(8)]
+        del held  # freed blocks of y's size, full of NaN
+        y = fs.flagsparse_spmv_coo(x=x, prepared=prepared)
+        # n products err by at most n * 2^-24 of their magnitude: 150 in the longest row here
+        assert bool(((y.double() - ref).abs() <= 1e-5 * ref).all())
