@@ -10,6 +10,14 @@ nonzeros, 40 held-out matrices above that, N in {1, 8, 32, 128}):
 
 which also trains and writes flagsparse_public_b200/selector_weights.npz.
 Then:  python tests/golden/make_selector_fixture.py sel_full.npz
+
+``selector_heldout_walk_times.npz`` holds the times of the same held-out
+samples, in the same order, on the present kernels (every candidate of the
+corpus timed again, 8 calls each; the weights stay):
+
+    python tests/golden/make_selector_fixture.py --times dataset.npz
+
+with a dataset of the arrays times, matrix and n_dense.
 """
 
 import os
@@ -32,5 +40,14 @@ def main(path):
                         names=z["names"])
 
 
+def times_only(path):
+    z = np.load(path, allow_pickle=False)
+    ref = np.load(os.path.join(HERE, "selector_heldout.npz"), allow_pickle=False)
+    at = {(int(m), int(n)): i for i, (m, n) in enumerate(zip(z["matrix"], z["n_dense"]))}
+    rows = [at[int(m), int(n)] for m, n in zip(ref["matrix"], ref["n_dense"])]
+    np.savez_compressed(os.path.join(HERE, "selector_heldout_walk_times.npz"),
+                        times=z["times"][rows].astype(np.float32), names=ref["names"])
+
+
 if __name__ == "__main__":
-    main(sys.argv[1])
+    times_only(sys.argv[2]) if sys.argv[1] == "--times" else main(sys.argv[1])
